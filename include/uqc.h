@@ -163,7 +163,8 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
 /* Launch tuning (no reference counterpart; the autotuner uses it):
  *   "closure_group"  threads per cell in the closure kernel: 32 (a warp per
  *                    cell, several cells per CTA), 64 (two warps per cell,
- *                    up to four cells per CTA) or 256 (a CTA per cell);
+ *                    up to four cells per CTA; the 2-D Euler closure: cells of
+ *                    a CTA iterating together) or 256 (a CTA per cell);
  *                    0 = automatic.
  *   "update_warps", "check_warps", "chord_warps"  warps (cells) per CTA of
  *                    the update kernel (default 8), the convergence-check
@@ -322,7 +323,8 @@ int uqc_closure_solve_device( uqc_solver* h, int n, double* d_lambda, const doub
  *
  * Precision: always the FP64 form, whatever the handle's precision (the mixed
  * form keeps a per-cell factor store, which would need an allocation); its
- * results are those of uqc_closure_solve_device on a UQC_FP64 handle.
+ * results are those of uqc_closure_solve_device on a UQC_FP64 handle (to
+ * rounding: the 2-D Euler closure runs another kernel there).
  *
  * Scratch lives in one statically allocated device array inside this library
  * (UQC_NOALLOC_SCRATCH_BYTES, held on every GPU that loads the library until

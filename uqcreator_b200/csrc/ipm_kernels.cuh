@@ -1,6 +1,7 @@
 // FP64 kernels of the IPM time step.
 //
-//   k_closure  persistent, work-stealing: one thread group (a warp for small
+//   k_closure  persistent, work-stealing (k_newton of newton_batch.cuh replaces
+//              it for the 2-D Euler closure): one thread group (a warp for small
 //              systems, a whole CTA for n = nS nT > 32) per cell. Runs the
 //              damped Newton of Closure::SolveClosure (closure.cpp:133-193) with
 //              the basis tables staged in shared memory, the Hessian kept in
@@ -32,7 +33,9 @@ constexpr int MAXLEV = 16;
 // gradient, 2 Hessian, 3 Cholesky, 4 back substitution, 5 trial gradients,
 // 6 epilogue, 7 load; chord Newton of the mixed form: 21 solves with the
 // held factor, 22 initial gradient, 23 whole cell, and counts 25 held-factor
-// directions, 26 refreshed factors, 27 trial gradients.
+// directions, 26 refreshed factors, 27 trial gradients; k_newton: 2 Hessian
+// product, 28 its scatter, 3 elimination, 4 back substitution, 5 trial, and the
+// count 29 of iterations.
 #ifdef UQC_PHASE_TIMERS
 #define PT_BEGIN( v ) long long v = clock64();
 #define PT_END( v, id ) \
@@ -106,6 +109,10 @@ struct KParams {
     const double* xi;        // nQ x dimXi
     const double* wt;        // nQ: w_k / 2^dimXi (phiWf = phi wt)
     const float* phiF;       // nQ x ld: phi rounded to FP32 (mixed form)
+    const double* phiT;      // nT x ldT: phi node-contiguous, zero from nQ to ldT (k_newton)
+    int ldT;                 // nQ rounded up to 4
+    int tabInSmem;           // k_newton: phiT staged in shared memory
+    const unsigned* pairSlots;    // k_newton: places of each (pair, block) in the Hessian tiles (low and high half)
     bool tablesInSmem;
     // geometry
     const double *area, *dx, *center, *unitN, *scaledN;

@@ -4,6 +4,7 @@
 #include "chord.cuh"
 #include "ipm_kernels.cuh"
 #include "kernels.h"
+#include "newton_batch.cuh"
 
 namespace uqc {
 
@@ -56,6 +57,17 @@ template <int CL> void* kernel_of( int group, int which ) {
             return nullptr;
 #endif
         }
+        case KERNEL_NEWTON_S4:
+        case KERNEL_NEWTON_S2:
+        case KERNEL_NEWTON_M2:
+        case KERNEL_NEWTON_L2:
+            if constexpr( CL == 1 ) {
+                if( which == KERNEL_NEWTON_S4 ) return (void*)&k_newton<CL, 4, 4, 2, 4>;
+                if( which == KERNEL_NEWTON_S2 ) return (void*)&k_newton<CL, 2, 4, 4, 4>;
+                if( which == KERNEL_NEWTON_M2 ) return (void*)&k_newton<CL, 2, 8, 4, 2>;
+                return (void*)&k_newton<CL, 2, 16, 5, 1>;
+            }
+            return nullptr;
         case KERNEL_CHORD:
         case KERNEL_HESS_TC:
         case KERNEL_INVERT_RAW:

@@ -38,18 +38,16 @@ __device__ unsigned long long g_phaseCycles[32];
 #define CT_END( v, id, cond )
 #endif
 
-// A thread group working on one cell: GROUP = 32 (a warp), 64 (two warps,
-// several groups per CTA, synchronised by named barrier `bar`) or the CTA.
+// A thread group working on one cell: GROUP = 32 (a warp) or several warps,
+// synchronised by named barrier `bar` (several groups may share a CTA).
 template <int GROUP> struct Grp {
     int r;      // rank in the group
-    int bar;    // named barrier id (GROUP == 64)
+    int bar;    // named barrier id, 1 .. 15 (GROUP > 32)
     __device__ __forceinline__ void sync() const {
         if constexpr( GROUP == 32 )
             __syncwarp();
-        else if constexpr( GROUP == 64 )
-            asm volatile( "bar.sync %0, 64;" ::"r"( bar ) : "memory" );
         else
-            __syncthreads();
+            asm volatile( "bar.sync %0, %1;" ::"r"( bar ), "n"( GROUP ) : "memory" );
     }
 };
 
@@ -120,11 +118,11 @@ __host__ __device__ inline size_t hess_doubles( int n ) {
     return nb * ( nb + 1 ) / 2 * 64 + nb * 8;
 }
 // in-tile offset of element (row k, column c)
-__device__ __forceinline__ int tix( int k, int c ) { return ( c << 3 ) | ( k ^ c ); }
-__device__ __forceinline__ int htile( int R, int C ) { return ( ( ( C * ( C + 1 ) ) >> 1 ) + R ) * 64; }
+__host__ __device__ __forceinline__ int tix( int k, int c ) { return ( c << 3 ) | ( k ^ c ); }
+__host__ __device__ __forceinline__ int htile( int R, int C ) { return ( ( ( C * ( C + 1 ) ) >> 1 ) + R ) * 64; }
 // offset of element (r, c), tile row r/8 <= tile column c/8
-__device__ __forceinline__ int hblk( int r, int c ) { return htile( r >> 3, c >> 3 ) + tix( r & 7, c & 7 ); }
-__device__ __forceinline__ int hrhs( int nb ) { return ( ( nb * ( nb + 1 ) ) >> 1 ) * 64; }
+__host__ __device__ __forceinline__ int hblk( int r, int c ) { return htile( r >> 3, c >> 3 ) + tix( r & 7, c & 7 ); }
+__host__ __device__ __forceinline__ int hrhs( int nb ) { return ( ( nb * ( nb + 1 ) ) >> 1 ) * 64; }
 
 // Upper-triangular pair index e -> (j, i), j <= i, column-major packed order.
 __device__ __forceinline__ void unpack_pair( int e, int& j, int& i ) {

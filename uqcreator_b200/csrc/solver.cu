@@ -28,6 +28,7 @@
 #include "chord.cuh"
 #include "ipm_kernels.cuh"
 #include "kernels.h"
+#include "newton_batch.cuh"
 #include "uqc.h"
 
 using namespace uqc;
@@ -49,6 +50,11 @@ struct uqc_solver {
     int chunkPartialCap    = 0;
     bool closureTiny = false;          // planned: the register Newton of tiny systems (k_closure TINY)
     int tinyGrid     = 0;
+    // FP64 closure of large systems: k_newton's instance (a KernelId, 0: k_closure) and launch shape
+    int newtonId = 0, newtonBlock = 0, newtonGrid = 0;
+    bool newtonTab = false;    // the basis table fits in shared memory beside the cells
+    size_t newtonSmem = 0;
+    unsigned* d_pairSlots = nullptr;    // k_newton: places of each (pair, block) value in the Hessian tiles
     size_t ldc = 1;
     // device buffers
     double *d_phi = nullptr, *d_phiWf = nullptr, *d_xi = nullptr;
@@ -79,6 +85,7 @@ struct uqc_solver {
     int closureTablesOpt     = -1;       // option closure_tables_smem: -1 automatic, 0 read through L1, 1 stage
     // mixed form: FP32 Hessian / factor / solves, FP64 gradient and update
     float* d_phiF        = nullptr;    // phi rounded to FP32, row stride ld
+    double* d_phiT       = nullptr;    // phi node-contiguous (nT rows of ldT), k_newton
     int* d_fallbackList  = nullptr;    // cells the mixed form hands to the FP64 form
     bool mixedOk         = false;
     std::string mixedWhy = "not planned";
@@ -265,6 +272,10 @@ KParams make_params( const uqc_solver* h ) {
     P.xi           = h->d_xi;
     P.wt           = h->d_wt;
     P.phiF         = h->d_phiF;
+    P.phiT         = h->d_phiT;
+    P.ldT          = ( h->tab.nQ + 3 ) & ~3;
+    P.pairSlots    = h->d_pairSlots;
+    P.tabInSmem    = h->newtonTab ? 1 : 0;
     P.tablesInSmem = h->tablesInSmem;
     P.area         = h->d_area;
     P.dx           = h->d_dx;
@@ -579,6 +590,63 @@ ClosureShape fp64_closure_shape( const uqc_solver* h, int maxSmem ) {
     return s;
 }
 
+// The batched Newton k_newton for the FP64 closure of the 2-D Euler states: the
+// first shape whose cells and CTAs per SM fit in shared memory and whose warps
+// hold a CTA's row tiles of 8 basis pairs. Small cells want many small CTAs
+// (one warp a cell; their phases overlap across the CTAs), large ones more
+// warps a cell. Closure phase of a step, k_closure / S4 / S2 / M2 / L2, where
+// a shape fits (us; 10-12 thousand unconverged cells of a 100k-cell mesh, and for
+// 84 and 140 duals 1.7 and 2.6 thousand):
+//   24 duals, 16 nodes     488 / 193 / 268 / 456 / 867
+//   40 duals, 36 nodes    1411 / 425 / 504 / 751 / 1396
+//   60 duals, 64 nodes    2818 /  -  / 1042 / 1333 / 2253
+//   84 duals, 100 nodes    861 /  -  /  -  / 430 / 562
+//   140 duals, 512 nodes 10528 /  -  /  -  /  -  / 3807
+// (12 duals: 336 -> 152 with 16 nodes, 530 -> 270 with 400.) Larger systems than
+// L2 holds stay with k_closure.
+void plan_newton( uqc_solver* h, int maxSmem ) {
+    h->newtonId  = 0;
+    const int cl = h->cfg.closure, nT = h->tab.nT, nQ = h->tab.nQ, nS = h->nS;
+    if( cl != 1 || ( h->closureGroupOverride != 0 && h->closureGroupOverride != 64 ) ) return;
+    const int tiles = ( nT * ( nT + 1 ) / 2 + 7 ) / 8;
+    struct Shape {
+        int id, cells, warps, rowTiles, ctas;    // the template arguments of k_newton
+    };
+    for( const Shape& s : {Shape{KERNEL_NEWTON_S4, 4, 4, 2, 4}, Shape{KERNEL_NEWTON_S2, 2, 4, 4, 4}, Shape{KERNEL_NEWTON_M2, 2, 8, 4, 2},
+                           Shape{KERNEL_NEWTON_L2, 2, 16, 5, 1}} ) {
+        const size_t cap   = size_t( maxSmem ) / s.ctas - ( s.ctas > 1 ? 1024 : 0 );
+        const size_t slots = ( size_t( s.cells ) * slot_layout( nS, nT, nQ, closure_np( cl ), 32 * s.warps / s.cells ).total + 4 ) * sizeof( double );
+        if( tiles > s.warps * s.rowTiles || slots > cap ) continue;
+        // the basis table beside the cells, or chunks of it in their nodal states
+        const size_t table = size_t( nT ) * ( ( ( nQ + 3 ) & ~3 ) | 4 ) * sizeof( double );
+        const bool staged  = slots + table <= cap;
+        const size_t smem  = slots + ( staged ? table : 0 );
+        if( !staged && newton_chunk( nS, nT, nQ ) == 0 ) continue;
+        void* fn = pick( cl, 32, s.id );
+        allow_dynamic_smem( fn );
+        int occ = 0;
+        CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, fn, 32 * s.warps, smem ) );
+        if( occ < 1 ) continue;
+        h->newtonId    = s.id;
+        h->newtonBlock = 32 * s.warps;
+        h->newtonGrid  = occ * h->numSMs;
+        h->newtonSmem  = smem;
+        h->newtonTab   = staged;
+        if( !h->d_pairSlots ) {
+            const int NP = closure_np( cl ), pairs = nT * ( nT + 1 ) / 2;
+            std::vector<unsigned> places( size_t( pairs ) * NP );
+            for( int p = 0; p < pairs; ++p )
+                for( int b = 0; b < NP; ++b ) {
+                    int row[2], col[2];
+                    pair_places( nS, p, b, nT, row, col );
+                    places[size_t( p ) * NP + b] = unsigned( rblk( row[0], col[0] ) ) | unsigned( rblk( row[1], col[1] ) ) << 16;
+                }
+            h->d_pairSlots = dupload( places );
+        }
+        return;
+    }
+}
+
 void plan_launches( uqc_solver* h ) {
     ++h->planGen;
     int dev;
@@ -673,6 +741,7 @@ void plan_launches( uqc_solver* h ) {
         CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kk, h->checkBlock, h->checkSmem ) );
         h->checkGrid = std::min( std::max( 1, occ ) * h->numSMs, std::max( 1, ( h->mesh.nCells + warps - 1 ) / warps ) );
     }
+    plan_newton( h, maxSmem );
     plan_mixed( h, maxSmem );
     plan_rounds( h, maxSmem );
 }
@@ -820,6 +889,11 @@ void ensure_device( uqc_solver* h ) {
     std::vector<float> phiF( phi.size() );
     for( size_t i = 0; i < phi.size(); ++i ) phiF[i] = float( phi[i] );
     h->d_phiF = dupload( phiF );
+    const int ldT = ( nQ + 3 ) & ~3;
+    std::vector<double> phiT( size_t( nT ) * ldT, 0.0 );
+    for( int k = 0; k < nQ; ++k )
+        for( int i = 0; i < nT; ++i ) phiT[size_t( i ) * ldT + k] = h->tab.phi[size_t( k ) * nT + i];
+    h->d_phiT = dupload( phiT );
     h->d_xi    = dupload( h->tab.xi );
     h->d_filter     = dupload( h->filterHost );
     h->d_lassoParam = dupload( h->lassoParamHost );
@@ -870,7 +944,7 @@ void release( uqc_solver* h ) {
                     (void*)h->d_unitN, (void*)h->d_scaledN, (void*)h->d_nbr, (void*)h->d_boundary, (void*)h->d_u, (void*)h->d_lam,
                     (void*)h->d_bndNormal, (void*)h->d_uQ, (void*)h->d_uOld0, (void*)h->d_blockPartial, (void*)h->d_chunkPartial, (void*)h->d_level, (void*)h->d_status,
                     (void*)h->d_iters, (void*)h->d_ctl, (void*)h->d_xLam, (void*)h->d_xU, (void*)h->d_xNt, (void*)h->d_xStatus,
-                    (void*)h->d_xIters, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_fallbackList,
+                    (void*)h->d_xIters, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_phiT, (void*)h->d_pairSlots, (void*)h->d_fallbackList,
                     (void*)h->d_factorStore, (void*)h->d_factorLevel, (void*)h->d_gStore, (void*)h->d_v2Lists,
                     (void*)h->d_chordIters, (void*)h->d_qTiles, (void*)h->d_sendCells, (void*)h->d_filter, (void*)h->d_lassoParam,
                     (void*)h->d_lassoL1} )
@@ -887,6 +961,19 @@ void release( uqc_solver* h ) {
     if( h->copyStreamOut ) cudaStreamDestroy( h->copyStreamOut );
     if( h->checkStream ) cudaStreamDestroy( h->checkStream );
     if( h->ownStream && h->stream ) cudaStreamDestroy( h->stream );
+}
+
+// The FP64 closure kernel over P's work list: k_newton where it is planned
+// (it runs SolveClosure's line-search Newton), else k_closure, which also runs
+// SolveClosureSafe and the One-Shot step.
+void launch_closure_fp64( uqc_solver* h, KParams& P, int mode ) {
+    void* args[] = {&P, &mode};
+    if( h->newtonId && P.newtonMode != 2 && P.maxIter > 1 ) {
+        launch( h, pick( h->cfg.closure, 32, h->newtonId ), h->newtonGrid, h->newtonBlock, h->newtonSmem, args );
+        return;
+    }
+    P.tablesInSmem = h->closureTablesInSmem;
+    launch( h, pick( h->cfg.closure, h->closureGroup, 0 ), h->closureGrid, h->closureBlock, h->closureSmem, args );
 }
 
 // Closure launch: the FP64 kernel; or the mixed-form kernel followed by the
@@ -944,16 +1031,12 @@ void launch_closure( uqc_solver* h, KParams& P, int mode ) {
         F.activeList  = h->d_fallbackList;
         F.activeCount = &h->d_ctl->nFallback;
         F.listParity  = 0;    // one fallback list
-        F.workCounter  = &h->d_ctl->workCounter2;
-        F.tablesInSmem = h->closureTablesInSmem;
-        void* fargs[]  = {&F, &mode};
-        launch( h, pick( h->cfg.closure, h->closureGroup, 0 ), h->closureGrid, h->closureBlock, h->closureSmem, fargs );
+        F.workCounter = &h->d_ctl->workCounter2;
+        launch_closure_fp64( h, F, mode );
         return;
     }
-    KParams Q      = P;
-    Q.tablesInSmem = h->closureTablesInSmem;
-    void* args[]   = {&Q, &mode};
-    launch( h, pick( h->cfg.closure, h->closureGroup, 0 ), h->closureGrid, h->closureBlock, h->closureSmem, args );
+    KParams Q = P;
+    launch_closure_fp64( h, Q, mode );
 }
 
 // Zeroes the closure work counters and the fallback list length (three
