@@ -52,7 +52,10 @@ enum uqc_layout { UQC_LAYOUT_REF = 0, UQC_LAYOUT_STATE_MAJOR = 1 };
  *            update stay FP64, so a converged cell meets the same FP64
  *            tolerance. Cells whose FP32 Newton does not converge (FP32
  *            factor not positive definite, line-search or iteration limit)
- *            continue from their last accepted duals in the FP64 form. */
+ *            continue from their last accepted duals in the FP64 form. Where
+ *            the FP64 form's kernel is the faster one it runs by default:
+ *            systems of at most 6 duals, the 2-D Euler closure of up to 48 duals
+ *            or without the tensor-core rounds, and its closure-only calls. */
 enum uqc_precision { UQC_FP64 = 0, UQC_MIXED = 1 };
 
 /* Per-cell closure status (uqc_cell_status). */
@@ -72,7 +75,7 @@ typedef struct uqc_info {
     double t;              /* simulated time */
     long long steps;       /* time steps taken */
     int mixed_form;        /* how UQC_MIXED time steps run the closure: 0 one kernel (FP32 Hessian on
-                              CUDA cores), 1 rounds of chord / Hessian / inverse kernels with the Hessian
+                              CUDA cores, or the FP64 form's where that is faster), 1 rounds of chord / Hessian / inverse kernels with the Hessian
                               on CUDA cores, 2 the same with the Hessian on the tensor cores; -1 before
                               the device side is set up (option "mixed_hessian") */
     int mixed_rounds;      /* re-factorisation rounds per time step of forms 1 and 2 */
@@ -208,8 +211,8 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
  *                    refinement level): -1 (default) rounds with the Hessian
  *                    on the tensor cores where its basis-pair table fits one
  *                    MMA (at most 256 pairs, i.e. total degree <= 5 in two
- *                    uncertainties), else the single kernel; 0 the single-kernel
- *                    form; 1 rounds with the CUDA-core Hessian; 2 rounds with
+ *                    uncertainties) and the system has more than 48 duals, else
+ *                    the FP64 form's kernel; 0 the single mixed kernel; 1 rounds with the CUDA-core Hessian; 2 rounds with
  *                    the tensor-core Hessian (UQC_ERR_CONFIG where it does
  *                    not fit). Rounds: a chord kernel (a warp per cell, held
  *                    inverse H0^-1 in FP32, FP64 gradients and tests), then

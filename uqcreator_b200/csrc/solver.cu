@@ -52,6 +52,9 @@ struct uqc_solver {
     int tinyGrid     = 0;
     // FP64 closure of large systems: k_newton's instance (a KernelId, 0: k_closure) and launch shape
     int newtonId = 0, newtonBlock = 0, newtonGrid = 0;
+    // UQC_MIXED runs k_newton (FP64) where it is faster than the mixed kernels: in
+    // time steps (mixedNewton) and in closure-only calls (mixedNewtonOnce)
+    bool mixedNewton = false, mixedNewtonOnce = false;
     bool newtonTab = false;    // the basis table fits in shared memory beside the cells
     size_t newtonSmem = 0;
     unsigned* d_pairSlots = nullptr;    // k_newton: places of each (pair, block) value in the Hessian tiles
@@ -303,7 +306,7 @@ KParams make_params( const uqc_solver* h ) {
     P.ctl           = h->d_ctl;
     P.workCounter   = h->d_ctl ? &h->d_ctl->workCounter : nullptr;
     P.fallbackList  = h->d_fallbackList;
-    const bool useStore = h->precision == UQC_MIXED && h->chord && h->d_factorStore;
+    const bool useStore = h->precision == UQC_MIXED && h->chord && !h->mixedNewton && h->d_factorStore;
     P.factorStore       = useStore ? h->d_factorStore : nullptr;
     P.factorLevel       = useStore ? h->d_factorLevel : nullptr;
     P.factorStride      = h->factorStride;
@@ -381,6 +384,7 @@ unsigned long long factor_store_bytes( const uqc_solver* h ) {
     const unsigned long long rounds = h->cfg.closure == 1 ? N * ( ( h->ldc + 2 + 3 ) / 4 * 4 * 8 + 4 * 4 ) : 0;
     return N * ( (unsigned long long)factor_stride( h ) * 4 + 4 ) + rounds;
 }
+void invalidate_lists( uqc_solver* h );
 // Allocates the store on first use; marks every stored factor invalid.
 void reset_factor_store( uqc_solver* h ) {
     const size_t N = size_t( h->mesh.nCells );
@@ -744,6 +748,23 @@ void plan_launches( uqc_solver* h ) {
     plan_newton( h, maxSmem );
     plan_mixed( h, maxSmem );
     plan_rounds( h, maxSmem );
+    // Which kernel the mixed form's default runs on the 2-D Euler closure. Steps:
+    // k_newton where the tensor-core rounds cannot run, and up to 48 duals, where
+    // a step's eight or ten launches and an FP32 inverse gain nothing; closure-only
+    // calls (no held inverse): always. Closure phase of a warm step, mixed kernels /
+    // k_newton (us): 24 duals, 10k cells 153 / 59, 100k cells 293 / 193; 40 duals
+    // 205 / 100 and 443 / 425; 60 duals 272 / 229 and 642 / 1036; 84 duals 387 /
+    // 430 and, on 200k cells, 1460 / 5080; without rounds: 80 duals, 216 nodes 968
+    // / 801; 140 duals, 512 nodes 4553 / 3816 (first step 34193 / 17540). Any option
+    // that asks for the mixed kernels' form keeps them.
+    const bool was     = h->mixedNewton;
+    h->mixedNewtonOnce = h->newtonId && h->mixedOk && h->roundsOpt == -1 && h->chord && h->mixedMaxIter == 0;
+    h->mixedNewton     = h->mixedNewtonOnce && ( h->v2Mode == 0 || n <= 48 );
+    if( h->deviceReady && h->precision == UQC_MIXED && was != h->mixedNewton ) {
+        // the mixed kernels need their store, and a next-step list with gradients
+        if( h->chord && !h->mixedNewton ) reset_factor_store( h );
+        invalidate_lists( h );
+    }
 }
 
 void reset_control( uqc_solver* h, double t ) {
@@ -932,7 +953,7 @@ void ensure_device( uqc_solver* h ) {
     for( auto& e : h->ev ) CK( cudaEventCreate( &e ) );
     plan_launches( h );
     if( h->precision == UQC_MIXED && !h->mixedOk ) throw ConfigError( "mixed precision not available for this configuration: " + h->mixedWhy );
-    if( h->precision == UQC_MIXED && h->chord ) reset_factor_store( h );
+    if( h->precision == UQC_MIXED && h->chord && !h->mixedNewton ) reset_factor_store( h );
     h->deviceReady = true;
     reset_control( h, 0.0 );
 }
@@ -1015,13 +1036,11 @@ void launch_closure( uqc_solver* h, KParams& P, int mode ) {
         F.activeCount  = &h->d_ctl->nFallback;
         F.listParity   = 0;
         F.workCounter  = &h->d_ctl->workCounter2;
-        F.tablesInSmem = h->closureTablesInSmem;
         F.gStore       = nullptr;
-        void* fargs[]  = {&F, &mode};
-        launch( h, pick( cl, h->closureGroup, 0 ), h->closureGrid, h->closureBlock, h->closureSmem, fargs );
+        launch_closure_fp64( h, F, mode );
         return;
     }
-    if( h->precision == UQC_MIXED && h->mixedOk ) {
+    if( h->precision == UQC_MIXED && h->mixedOk && !( ( mode == 1 ? h->mixedNewton : h->mixedNewtonOnce ) && P.newtonMode != 2 && P.maxIter > 1 ) ) {
         KParams M      = P;
         M.tablesInSmem = h->mixedTablesInSmem;
         if( h->mixedMaxIter > 1 && P.maxIter > 1 ) M.maxIter = std::min( P.maxIter, h->mixedMaxIter );
@@ -1166,7 +1185,9 @@ unsigned long long device_bytes_of( const uqc_solver* h ) {
     const unsigned long long tab = ( (unsigned long long)h->tab.nQ * h->ld + 8 ) * ( 8 + 8 + 4 ) + h->tab.xi.size() * 8 + h->tab.nQ * 8;
     const unsigned long long d8  = N * ( 3 * ldc + 1 + 1 + 1 + 2 + 4 * F ) + ( N + 1 ) * sq;    // state (u, re-projected u, lambda), uQ, geometry, cell dt
     const unsigned long long d4  = N * ( F + 1 + 1 + 1 + 1 + 2 + 2 + 1 );                     // nbr, boundary, level, status, iters, lists
-    return tab + 8 * d8 + 4 * d4 + N + ( mesh_has_walls( h->mesh ) ? 16 * N : 0 ) + sizeof( Control ) + 8 * 4096 + ( h->precision == UQC_MIXED && h->chord ? factor_store_bytes( h ) : 0 );
+    return tab + 8 * d8 + 4 * d4 + N + ( mesh_has_walls( h->mesh ) ? 16 * N : 0 ) + sizeof( Control ) + 8 * 4096 + 
+           // (counted before the device side is set up even where the default then runs without the store)
+           ( h->precision == UQC_MIXED && h->chord && !( h->deviceReady && !h->d_factorStore ) ? factor_store_bytes( h ) : 0 );
 }
 
 void to_layout( const uqc_solver* h, const double* src, double* dst, int layout, bool toDevice ) {
@@ -1291,7 +1312,7 @@ int uqc_get_info( const uqc_solver* h, uqc_info* o ) {
     o->newton_mode = h->cfg.newtonMode;
     o->t           = h->h_ctl ? h->h_ctl->t : 0.0;
     o->steps       = h->h_ctl ? h->h_ctl->steps : 0;
-    o->mixed_form  = h->deviceReady ? h->v2Mode : -1;
+    o->mixed_form  = h->deviceReady ? ( h->mixedNewton ? 0 : h->v2Mode ) : -1;
     o->mixed_rounds = h->v2Rounds;
     return UQC_OK;
 }
@@ -1304,7 +1325,7 @@ int uqc_set_precision( uqc_solver* h, int precision ) {
     } );
     if( rc != UQC_OK ) return rc;
     if( precision == UQC_MIXED && !h->mixedOk ) return fail( h, UQC_ERR_CONFIG, "mixed precision not available for this configuration: " + h->mixedWhy );
-    if( precision == UQC_MIXED && h->chord ) {
+    if( precision == UQC_MIXED && h->chord && !h->mixedNewton ) {
         rc = guarded( h, [&] {
             reset_factor_store( h );
             return UQC_OK;
@@ -1371,6 +1392,10 @@ int uqc_set_option( uqc_solver* h, const char* key, double value ) {
         if( v != 0 && v < 2 ) return fail( h, UQC_ERR_ARGUMENT, "mixed_max_iterations must be 0 or >= 2" );
         h->mixedMaxIter = v;
         ++h->planGen;
+        if( h->deviceReady ) return guarded( h, [&] {
+                plan_launches( h );
+                return UQC_OK;
+            } );
         return UQC_OK;
     }
     if( k == "mixed_chord" || k == "mixed_chord_inverse" ) {
@@ -1378,7 +1403,7 @@ int uqc_set_option( uqc_solver* h, const char* key, double value ) {
         if( h->deviceReady ) {
             int rc = guarded( h, [&] {
                 plan_launches( h );    // the mixed workspace depends on the chord form
-                if( h->chord && h->precision == UQC_MIXED ) reset_factor_store( h );
+                if( h->chord && h->precision == UQC_MIXED && !h->mixedNewton ) reset_factor_store( h );
                 return UQC_OK;
             } );
             if( rc != UQC_OK ) return rc;
@@ -1394,7 +1419,7 @@ int uqc_set_option( uqc_solver* h, const char* key, double value ) {
         if( h->deviceReady ) {
             int rc = guarded( h, [&] {
                 plan_launches( h );
-                if( h->chord && h->precision == UQC_MIXED ) reset_factor_store( h );    // the store's format depends on the form
+                if( h->chord && h->precision == UQC_MIXED && !h->mixedNewton ) reset_factor_store( h );    // the store's format depends on the form
                 invalidate_lists( h );    // the next step's list carries no stored gradients yet
                 return UQC_OK;
             } );
