@@ -1,5 +1,4 @@
-"""k_newton, the FP64 closure whose cells iterate together (2-D Euler): every
-launch shape and the remainders of its tiles (basis pairs in eights, duals in
+"""k_newton, the FP64 closure whose cells iterate together: every launch shape and the remainders of its tiles (basis pairs in eights, duals in
 eights, nodes in fours), against the FP64 oracle."""
 import numpy as np
 import pytest
@@ -59,6 +58,35 @@ def test_closure_of_a_batch(degree, nquad, dim_xi, n):
     ok = status == 0
     rounding = 8 * nquad ** dim_xi * np.finfo(float).eps * np.linalg.norm(u.reshape(n, -1), axis=1)
     assert np.all(_residual(o, lam[ok], u[ok]) < EPS + rounding[ok])
+
+
+@pytest.mark.parametrize("toml", [
+    W.burgers1d(ncells=90, degree=6, nquad=9, eps=EPS),      # 7 duals: more than the register Newton takes
+    W.burgers1d(ncells=90, degree=9, nquad=40, eps=EPS),     # 55 pairs, 7 row tiles
+    W.burgers1d(ncells=90, degree=10, nquad=21, eps=EPS),    # 66 pairs: the second shape
+    W.burgers1d(ncells=90, degree=14, nquad=30, eps=EPS),    # 120 pairs, its largest
+    W.shallow_water1d(ncells=90, max_degree=3, nquad=7, eps=EPS),
+    W.shallow_water1d(ncells=90, max_degree=9, nquad=30, eps=EPS),
+], ids=["burgers_7", "burgers_10", "burgers_11", "burgers_15", "sw_8", "sw_20"])
+def test_closure_of_small_systems(toml):
+    """One and two states, odd numbers of blocks: statuses and the convergence
+    test as above, with different moment counts per cell where there are levels."""
+    o, s = Oracle(toml), Solver(toml)
+    o.init_state()
+    u, lam0, _ = o.get_state()
+    nt = np.array(s.n_total_levels, dtype=np.uint32)[np.arange(len(u)) % s.n_levels]
+    for j, t in enumerate(nt):
+        u[j, :, t:] = 0.0
+    lam, status = s.closure_solve_host(lam0, u, nt)
+    _, expect_status = o.solve_closure(lam0.copy(), u, nt)[:2]
+    np.testing.assert_array_equal(status, expect_status)
+    phi, phi_wf = o.tables()[:2]
+    for j in np.nonzero(status == 0)[0]:
+        t = nt[j]
+        uk = np.stack([o.ansatz(lam[j, :, :t] @ phi[k, :t])[0] for k in range(phi.shape[0])], 1)
+        rounding = 8 * phi.shape[0] * np.finfo(float).eps * np.linalg.norm(u[j])
+        assert np.linalg.norm(uk @ phi_wf[:, :t] - u[j, :, :t]) < EPS + rounding
+    assert np.count_nonzero(status == 0) > len(u) // 2
 
 
 @pytest.mark.parametrize("degree,nquad,dim_xi", [(1, 2, 2), (3, 5, 2), (4, 7, 2), (4, 5, 3)])

@@ -67,6 +67,10 @@ template <int CL> void* kernel_of( int group, int which ) {
                 if( which == KERNEL_NEWTON_M2 ) return (void*)&k_newton<CL, 2, 8, 4, 2>;
                 return (void*)&k_newton<CL, 2, 16, 5, 1>;
             }
+            else if constexpr( !Closure<CL>::LINEAR ) {
+                if( which == KERNEL_NEWTON_S4 ) return (void*)&k_newton<CL, 4, 4, 2, 4>;
+                if( which == KERNEL_NEWTON_S2 ) return (void*)&k_newton<CL, 2, 4, 4, 4>;
+            }
             return nullptr;
         case KERNEL_CHORD:
         case KERNEL_HESS_TC:

@@ -1,4 +1,4 @@
-// FP64 Newton closure of the 2-D Euler states (k_newton): several cells share a
+// FP64 Newton closure (k_newton): several cells share a
 // CTA and take their Newton iterations together.
 //
 // An iteration of Closure::SolveClosure (closure.cpp:133-193) on a cell of
@@ -330,7 +330,6 @@ template <int CL, int B, int W, int MQ, int CTAS>
 __global__ void __launch_bounds__( 32 * W, CTAS ) k_newton( KParams P, int mode ) {
     constexpr int NS = Closure<CL>::NS, NP = Closure<CL>::NP, G = W / B, GROUP = 32 * G, NT = ( NP * B + 7 ) / 8;
     static_assert( B >= 2, "the table's chunks use two slots' nodal states" );
-    static_assert( NP % 2 == 0, "accumulator column pairs stay within a cell's blocks" );
     extern __shared__ __align__( 16 ) double smem[];
     if( mode == 1 && !P.ctl->active ) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slot = warp / G;
@@ -405,7 +404,12 @@ __global__ void __launch_bounds__( 32 * W, CTAS ) k_newton( KParams P, int mode 
 #pragma unroll
                     for( int s = 0; s < NS; ++s ) L[s] = fma( li[s], r, L[s] );
                 }
-                Closure<CL>::UDU( L, u, y, P.phys );
+                if constexpr( CL == 1 )
+                    Closure<CL>::UDU( L, u, y, P.phys );
+                else {
+                    Closure<CL>::U( L, u, true, P.phys );
+                    Closure<CL>::DU( L, y, P.phys );
+                }
                 const double w = __ldg( P.wt + k );
 #pragma unroll
                 for( int s = 0; s < NS; ++s ) uk[k * NS + s] = u[s];
@@ -585,22 +589,22 @@ __global__ void __launch_bounds__( 32 * W, CTAS ) k_newton( KParams P, int mode 
                 if( p >= pairs ) continue;
 #pragma unroll
                 for( int nt = 0; nt < NT; ++nt ) {
-                    const int col = 8 * nt + 2 * t;    // two columns: blocks b and b + 1 of a slot (NP is even)
-                    if( col >= NP * B ) continue;
-                    const int sl = col / NP, b = col - sl * NP;
-                    double* Hs   = smem + size_t( sl ) * S.total + S.hd;
-                    if( uniform || nTs[sl] == P.nT ) {
-                        // both places of each value from the table (the same one twice
-                        // for a value that is not mirrored)
-                        const uint2 o     = __ldg( reinterpret_cast<const uint2*>( P.pairSlots + p * NP + b ) );
-                        Hs[o.x & 0xFFFFu] = acc[q][nt][0];
-                        Hs[o.x >> 16]     = acc[q][nt][0];
-                        Hs[o.y & 0xFFFFu] = acc[q][nt][1];
-                        Hs[o.y >> 16]     = acc[q][nt][1];
-                    }
-                    else if( nTs[sl] > 0 ) {
-                        scatter_value<NS>( Hs, p, b, nTs[sl], acc[q][nt][0] );
-                        scatter_value<NS>( Hs, p, b + 1, nTs[sl], acc[q][nt][1] );
+                    // two adjacent columns: blocks of the same slot when NP is even
+#pragma unroll
+                    for( int h = 0; h < 2; ++h ) {
+                        const int col = 8 * nt + 2 * t + h;
+                        if( col >= NP * B ) continue;
+                        const int sl = col / NP, b = col - sl * NP;
+                        double* Hs   = smem + size_t( sl ) * S.total + S.hd;
+                        if( uniform || nTs[sl] == P.nT ) {
+                            // both places of the value from the table (the same one twice
+                            // for a value that is not mirrored)
+                            const unsigned o = __ldg( P.pairSlots + p * NP + b );
+                            Hs[o & 0xFFFFu]  = acc[q][nt][h];
+                            Hs[o >> 16]      = acc[q][nt][h];
+                        }
+                        else if( nTs[sl] > 0 )
+                            scatter_value<NS>( Hs, p, b, nTs[sl], acc[q][nt][h] );
                     }
                 }
             }

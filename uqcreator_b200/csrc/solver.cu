@@ -594,24 +594,27 @@ ClosureShape fp64_closure_shape( const uqc_solver* h, int maxSmem ) {
     return s;
 }
 
-// The batched Newton k_newton for the FP64 closure of the 2-D Euler states: the
-// first shape whose cells and CTAs per SM fit in shared memory and whose warps
-// hold a CTA's row tiles of 8 basis pairs. Small cells want many small CTAs
-// (one warp a cell; their phases overlap across the CTAs), large ones more
-// warps a cell. Closure phase of a step, k_closure / S4 / S2 / M2 / L2, where
-// a shape fits (us; 10-12 thousand unconverged cells of a 100k-cell mesh, and for
-// 84 and 140 duals 1.7 and 2.6 thousand):
+// The batched Newton k_newton for the FP64 closure: the first shape whose cells
+// and CTAs per SM fit in shared memory and whose warps hold a CTA's row tiles
+// of 8 basis pairs. Small cells want many small CTAs (one warp a cell; their
+// phases overlap across the CTAs), large ones more warps a cell. Closure phase
+// of a 2-D Euler step, k_closure / S4 / S2 / M2 / L2, where a shape fits (us; 10-12
+// thousand unconverged cells of a 100k-cell mesh, and for 84 and 140 duals 1.7
+// and 2.6 thousand):
 //   24 duals, 16 nodes     488 / 193 / 268 / 456 / 867
 //   40 duals, 36 nodes    1411 / 425 / 504 / 751 / 1396
 //   60 duals, 64 nodes    2818 /  -  / 1042 / 1333 / 2253
 //   84 duals, 100 nodes    861 /  -  /  -  / 430 / 562
 //   140 duals, 512 nodes 10528 /  -  /  -  /  -  / 3807
-// (12 duals: 336 -> 152 with 16 nodes, 530 -> 270 with 400.) Larger systems than
-// L2 holds stay with k_closure.
+// (12 duals: 336 -> 152 with 16 nodes, 530 -> 270 with 400.) Fewer states, k_closure
+// / S4: Burgers, 10 duals, 20k cells 106 / 68, 500 cells 64 / 51, first step
+// 1354 / 585; adaptive shallow water, 1M cells, first step 9478 / 4854; 1-D
+// Euler, 15 duals, 94 / 72, 45 duals (S2) 249 / 138. Larger systems than L2
+// holds stay with k_closure.
 void plan_newton( uqc_solver* h, int maxSmem ) {
     h->newtonId  = 0;
     const int cl = h->cfg.closure, nT = h->tab.nT, nQ = h->tab.nQ, nS = h->nS;
-    if( cl != 1 || ( h->closureGroupOverride != 0 && h->closureGroupOverride != 64 ) ) return;
+    if( closure_linear( cl ) || ( h->closureGroupOverride != 0 && h->closureGroupOverride != 64 ) ) return;
     const int tiles = ( nT * ( nT + 1 ) / 2 + 7 ) / 8;
     struct Shape {
         int id, cells, warps, rowTiles, ctas;    // the template arguments of k_newton
@@ -626,6 +629,7 @@ void plan_newton( uqc_solver* h, int maxSmem ) {
         const bool staged  = slots + table <= cap;
         const size_t smem  = slots + ( staged ? table : 0 );
         if( !staged && newton_chunk( nS, nT, nQ ) == 0 ) continue;
+        if( cl != 1 && s.id != KERNEL_NEWTON_S4 && s.id != KERNEL_NEWTON_S2 ) continue;    // the shapes built for every closure
         void* fn = pick( cl, 32, s.id );
         allow_dynamic_smem( fn );
         int occ = 0;
