@@ -1,0 +1,60 @@
+"""The check and update kernels of cells with few moments: several lanes per
+cell, instances of 6, 10 and 16 moments; cell counts that leave a warp partly
+empty, node counts that leave lanes idle, with and without the next step's
+test, against the FP64 oracle."""
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle
+from uqcreator_b200 import workloads as W
+from uqcreator_b200.solver import Solver
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "burgers_3_cells": W.burgers1d(ncells=3, degree=4, nquad=20, tend=10.0),
+    "burgers_2_moments": W.burgers1d(ncells=37, degree=1, nquad=3, tend=10.0),
+    "burgers_6_moments": W.burgers1d(ncells=65, degree=5, nquad=17, tend=10.0),
+    "burgers_7_moments": W.burgers1d(ncells=41, degree=6, nquad=9, tend=10.0),
+    "burgers_16_moments": W.burgers1d(ncells=43, degree=15, nquad=33, tend=10.0),
+    "burgers_17_moments": W.burgers1d(ncells=43, degree=16, nquad=35, tend=10.0),    # the warp-per-cell kernels
+    "sw_levels": W.shallow_water1d(ncells=131, max_degree=9, nquad=30, tend=10.0),
+    "sw_16_moments": W.shallow_water1d(ncells=70, max_degree=15, nquad=32, tend=10.0),
+    "euler_3_moments": W.euler2d(nx=7, ny=3, degree=1, nquad=3, tend=10.0),
+    "euler_6_moments": W.euler2d(nx=16, ny=5, degree=2, nquad=5, tend=10.0),
+}
+
+
+@pytest.mark.parametrize("update_test", [0, 1])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_steps_match_oracle(name, update_test):
+    """Moments within 1e-9 of their largest, equal levels, dt, residual and failed
+    cells. (Not the relative error of E and Var: three cells keep a state
+    without variance, whose relative error compares rounding with rounding.)"""
+    toml = CASES[name]
+    s, o = Solver(toml), Oracle(toml, W.mesh_for(toml))
+    s.set_option("update_test", update_test)
+    s.init_state()
+    o.init_state()
+    a, b = s.step(9), o.step(9)
+    assert a["steps"] == 9 and a["failed_cells"] == b["failures"]
+    assert a["dt"] == pytest.approx(b["dt"], rel=1e-12) and a["residual"] == pytest.approx(b["residual"], rel=1e-9, abs=1e-15)
+    us, _, vs = s.download_state()
+    uo, _, vo = o.get_state()
+    np.testing.assert_array_equal(vs, vo)
+    np.testing.assert_allclose(us, uo, rtol=0, atol=1e-9 * np.abs(uo).max())
+
+
+def test_large_mesh_of_ten_moments():
+    """2-D Euler with 10 moments takes these kernels only from 20,000 cells on:
+    its two instances (option update_test) against each other."""
+    toml = W.euler2d(nx=120, ny=90, degree=3, nquad=6, tend=10.0)
+    out = []
+    for v in (0, 1):
+        s = Solver(toml)
+        s.set_option("update_test", v)
+        s.init_state()
+        s.step(3)
+        out.append(s.download_state()[0])
+        s.close()
+    np.testing.assert_allclose(out[0], out[1], rtol=0, atol=1e-9 * np.abs(out[0]).max())

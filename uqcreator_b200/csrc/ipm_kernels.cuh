@@ -1514,6 +1514,65 @@ __device__ __forceinline__ void finish_cell( const KParams& P, int cell, double 
     dtNext         = d < dtNext ? d : dtNext;
 }
 
+// End of an update kernel, by every CTA: the CTA's part of the residual (res per
+// thread), and in the last CTA to arrive the residual of the step and the loop
+// control. The sums have a fixed order: per thread, warp and CTA, then over the
+// CTAs by 32 lanes in turn (lane l: CTAs l, l + 32, ...) and a butterfly.
+__device__ __forceinline__ void update_epilogue( const KParams& P, double res, double dt, bool finish ) {
+    __shared__ double blockRes[32];
+    __shared__ int isLast;
+    for( int o = 16; o > 0; o >>= 1 ) res += __shfl_xor_sync( 0xffffffffu, res, o );
+    if( ( threadIdx.x & 31 ) == 0 ) blockRes[threadIdx.x >> 5] = res;
+    __syncthreads();
+    if( threadIdx.x == 0 ) {
+        double s = 0.0;
+        for( int w = 0; w < int( blockDim.x >> 5 ); ++w ) s += blockRes[w];
+        P.blockPartial[size_t( P.updChunk ) * gridDim.x + blockIdx.x] = s;
+        __threadfence();
+        unsigned done = atomicAdd( &P.ctl->doneBlocks, 1u );
+        // the launches of a chunked update run one after another on the
+        // stream: the last CTA of the last launch finishes the step
+        isLast = done == gridDim.x * unsigned( P.updChunks ) - 1;
+    }
+    __syncthreads();
+    double total = 0.0;
+    if( isLast && threadIdx.x < 32 ) {
+        __threadfence();
+        const unsigned nb = gridDim.x * unsigned( P.updChunks );
+        for( unsigned b = threadIdx.x; b < nb; b += 32 ) total += ( (volatile double*)P.blockPartial )[b];
+        for( int o = 16; o > 0; o >>= 1 ) total += __shfl_xor_sync( 0xffffffffu, total, o );
+    }
+    if( isLast && threadIdx.x == 0 ) {
+        Control* C    = P.ctl;
+        C->nActive[C->steps & 1] = 0;    // this step's lists are consumed (before steps advances)
+        C->nCheck[C->steps & 1]  = 0;
+        C->residual   = total;
+        C->dt         = dt;
+        C->t          = C->t + dt;
+        C->steps      = C->steps + 1;
+        C->active     = ( C->t < C->tEnd && C->residual > C->minResidual && ( C->maxSteps == 0 || C->steps < C->maxSteps ) ) ? 1 : 0;
+        C->activeCellsLast = C->activeCells;
+        C->activeCells     = 0;
+        // retardation: raise the level cap as the residual falls below the thresholds
+        if( P.nRet > 0 ) {
+            int k = C->retIndex;
+            while( k < P.nRet && total < P.retRes[k] ) ++k;
+            C->retIndex = k;
+            C->levelCap = P.retLev[k];
+        }
+        // the next step's min starts from the cells finished here (+inf if none)
+        C->dtBits     = finish ? ( (volatile unsigned long long*)&C->dtBitsNext )[0] : 0x7FF0000000000000ull;
+        C->dtBitsNext = 0x7FF0000000000000ull;
+        C->listReady = finish ? 1 : 0;
+        C->workCounter  = 0;
+        C->workCounter2 = 0;
+        C->nFallback    = 0;
+        for( int r = 0; r < 16; ++r ) C->v2Work[r] = 0;
+        for( int r = 0; r < 4; ++r ) C->v2Count[r] = 0;
+        C->doneBlocks  = 0;
+    }
+}
+
 // Flux + explicit Euler update (expliciteuler.cpp:17-74), one warp per cell
 // (grid-stride over cells, many warps per SM), and the residual / time
 // control finished by the last CTA. Per node the kinetic fluxes of the cell's
@@ -1544,8 +1603,6 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
     const bool finish = FIN && P.finishInUpdate;
     constexpr int NS = Closure<CL>::NS;
     extern __shared__ __align__( 16 ) double smem[];
-    __shared__ double blockRes[32];
-    __shared__ int isLast;
     if( !P.ctl->active ) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nWarps = blockDim.x >> 5;
     const double* phiWf = P.phiWf;
@@ -1638,17 +1695,18 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
                     a[s]    = ua[s * P.nQ + k];
                     gsum[s] = 0.0;
                 }
+                const typename Problem<CL>::Side sa = Problem<CL>::side( a, P.phys.gamma );
                 if( wall ) wall_ghost<CL>( a, bn, bc == 2, gh );
 #pragma unroll
                 for( int f = 0; f < 3; ++f ) {
                     if( f < P.nFaces ) {
                         double b[NS], y[NS];
                         if( ghost[f] )
-                            Problem<CL>::flux( gh, gh, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y, P.phys );
+                            Problem<CL>::flux( gh, Problem<CL>::side( gh, P.phys.gamma ), gh, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y, P.phys );
                         else {
 #pragma unroll
                             for( int s = 0; s < NS; ++s ) b[s] = ub[f][s * P.nQ + k];
-                            Problem<CL>::flux( a, b, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y, P.phys );
+                            Problem<CL>::flux( a, sa, b, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y, P.phys );
                         }
 #pragma unroll
                         for( int s = 0; s < NS; ++s ) gsum[s] += y[s];
@@ -1671,6 +1729,7 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
                     a1[s] = ua[s * P.nQ + k1];
                     g0[s] = g1[s] = 0.0;
                 }
+                const typename Problem<CL>::Side sa0 = Problem<CL>::side( a0, P.phys.gamma ), sa1 = Problem<CL>::side( a1, P.phys.gamma );
 #pragma unroll
                 for( int f = 0; f < 3; ++f ) {
                     if( f < P.nFaces ) {
@@ -1680,8 +1739,8 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
                             b0[s] = ub[f][s * P.nQ + k0];
                             b1[s] = ub[f][s * P.nQ + k1];
                         }
-                        Problem<CL>::flux( a0, b0, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y0, P.phys );
-                        Problem<CL>::flux( a1, b1, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y1, P.phys );
+                        Problem<CL>::flux( a0, sa0, b0, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y0, P.phys );
+                        Problem<CL>::flux( a1, sa1, b1, fd + 5 * f, fd + 5 * f + 2, fd[5 * f + 4], y1, P.phys );
 #pragma unroll
                         for( int s = 0; s < NS; ++s ) {
                             g0[s] += y0[s];
@@ -1719,8 +1778,8 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
                         b0[s] = n0[s * P.nQ + k0];
                         b1[s] = n1[s * P.nQ + k1];
                     }
-                    Problem<CL>::flux( a0, b0, fd + 5 * f0, fd + 5 * f0 + 2, fd[5 * f0 + 4], y0, P.phys );
-                    Problem<CL>::flux( a1, b1, fd + 5 * f1, fd + 5 * f1 + 2, fd[5 * f1 + 4], y1, P.phys );
+                    Problem<CL>::flux( a0, Problem<CL>::side( a0, P.phys.gamma ), b0, fd + 5 * f0, fd + 5 * f0 + 2, fd[5 * f0 + 4], y0, P.phys );
+                    Problem<CL>::flux( a1, Problem<CL>::side( a1, P.phys.gamma ), b1, fd + 5 * f1, fd + 5 * f1 + 2, fd[5 * f1 + 4], y1, P.phys );
 #pragma unroll
                     for( int s = 0; s < NS; ++s ) Yt[j0 * NS + s] = y0[s];
                     if( two ) {
@@ -1850,63 +1909,7 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
         cbuf.flush( lane, clist, ccount );
     }
     if( lane == 0 && dtNext < 1e300 ) atomic_min_pos_double( &P.ctl->dtBitsNext, dtNext );
-    // deterministic residual: per-thread partials -> CTA sum -> per-CTA slot -> last CTA sums in order
-    for( int o = 16; o > 0; o >>= 1 ) res += __shfl_xor_sync( 0xffffffffu, res, o );
-    if( ( threadIdx.x & 31 ) == 0 ) blockRes[threadIdx.x >> 5] = res;
-    __syncthreads();
-    if( threadIdx.x == 0 ) {
-        double s = 0.0;
-        for( int w = 0; w < int( blockDim.x >> 5 ); ++w ) s += blockRes[w];
-        P.blockPartial[size_t( P.updChunk ) * gridDim.x + blockIdx.x] = s;
-        __threadfence();
-        unsigned done = atomicAdd( &P.ctl->doneBlocks, 1u );
-        // the launches of a chunked update run one after another on the
-        // stream: the last CTA of the last launch finishes the step
-        isLast = done == gridDim.x * unsigned( P.updChunks ) - 1;
-    }
-    __syncthreads();
-    double total = 0.0;
-    if( isLast && threadIdx.x < 32 ) {
-        __threadfence();
-        // the CTA partials in launch and CTA order: the warp loads 32 at a
-        // time, lane 0 adds them in sequence from the shuffles
-        const unsigned nb = gridDim.x * unsigned( P.updChunks );
-        for( unsigned b0 = 0; b0 < nb; b0 += 32 ) {
-            const unsigned b = b0 + threadIdx.x;
-            const double v   = b < nb ? ( (volatile double*)P.blockPartial )[b] : 0.0;
-            const unsigned m = min( 32u, nb - b0 );
-            for( unsigned j = 0; j < m; ++j ) total += __shfl_sync( 0xffffffffu, v, int( j ) );
-        }
-    }
-    if( isLast && threadIdx.x == 0 ) {
-        Control* C    = P.ctl;
-        C->nActive[C->steps & 1] = 0;    // this step's lists are consumed (before steps advances)
-        C->nCheck[C->steps & 1]  = 0;
-        C->residual   = total;
-        C->dt         = dt;
-        C->t          = C->t + dt;
-        C->steps      = C->steps + 1;
-        C->active     = ( C->t < C->tEnd && C->residual > C->minResidual && ( C->maxSteps == 0 || C->steps < C->maxSteps ) ) ? 1 : 0;
-        C->activeCellsLast = C->activeCells;
-        C->activeCells     = 0;
-        // retardation: raise the level cap as the residual falls below the thresholds
-        if( P.nRet > 0 ) {
-            int k = C->retIndex;
-            while( k < P.nRet && total < P.retRes[k] ) ++k;
-            C->retIndex = k;
-            C->levelCap = P.retLev[k];
-        }
-        // the next step's min starts from the cells finished here (+inf if none)
-        C->dtBits     = finish ? ( (volatile unsigned long long*)&C->dtBitsNext )[0] : 0x7FF0000000000000ull;
-        C->dtBitsNext = 0x7FF0000000000000ull;
-        C->listReady = finish ? 1 : 0;
-        C->workCounter  = 0;
-        C->workCounter2 = 0;
-        C->nFallback    = 0;
-        for( int r = 0; r < 16; ++r ) C->v2Work[r] = 0;
-        for( int r = 0; r < 4; ++r ) C->v2Count[r] = 0;
-        C->doneBlocks  = 0;
-    }
+    update_epilogue( P, res, dt, finish );
 }
 
 // Initial moments u_j = U_IC(x_j, xi_k) phiWf and duals lambda_j(:,0) = DS(u_j(:,0)).

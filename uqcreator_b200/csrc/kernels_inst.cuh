@@ -5,8 +5,21 @@
 #include "ipm_kernels.cuh"
 #include "kernels.h"
 #include "newton_batch.cuh"
+#include "small_cells.cuh"
 
 namespace uqc {
+
+// The instances for few moments: NTM = 6, 10 or 16, as far as a lane's registers
+// hold a cell's sums.
+template <int CL, int NTM> void* small_kernel_of( int which ) {
+    if constexpr( Closure<CL>::NS * NTM <= 40 ) {
+        if constexpr( !Closure<CL>::LINEAR && Closure<CL>::NS < 4 )
+            if( which == KERNEL_CHECK_SMALL ) return (void*)&k_check_small<CL, NTM>;
+        if( which == KERNEL_UPDATE_SMALL ) return (void*)&k_update_small<CL, true, NTM>;
+        if( which == KERNEL_UPDATE_SMALL_PLAIN ) return (void*)&k_update_small<CL, false, NTM>;
+    }
+    return nullptr;
+}
 
 template <int CL> void* kernel_of( int group, int which ) {
     if constexpr( Closure<CL>::LINEAR ) {
@@ -49,6 +62,13 @@ template <int CL> void* kernel_of( int group, int which ) {
             if( group == 256 ) return (void*)&k_meanvar<CL, 256>;
             return nullptr;
         case KERNEL_CHECK: return (void*)&k_check<CL>;
+        case KERNEL_CHECK_SMALL:
+        case KERNEL_UPDATE_SMALL:
+        case KERNEL_UPDATE_SMALL_PLAIN:
+            if( group == SMALL_NT[0] ) return small_kernel_of<CL, SMALL_NT[0]>( which );
+            if( group == SMALL_NT[1] ) return small_kernel_of<CL, SMALL_NT[1]>( which );
+            if( group == SMALL_NT[2] ) return small_kernel_of<CL, SMALL_NT[2]>( which );
+            return nullptr;
         case KERNEL_PHASE_COUNTERS: {
 #ifdef UQC_PHASE_TIMERS
             void* p = nullptr;

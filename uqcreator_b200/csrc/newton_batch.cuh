@@ -87,16 +87,6 @@ __host__ __device__ inline int newton_chunk( int nS, int nT, int nQ ) {
     return fit < 4 ? 0 : fit - ( fit + 4 ) % 8;
 }
 
-// 1/d: the PTX FP64 reciprocal estimate (about 20 bits) refined by the
-// third-order iteration r (1 + e + e^2), e = 1 - d r, which cubes the relative
-// error (to rounding).
-__device__ __forceinline__ double reciprocal( double d ) {
-    double r;
-    asm( "rcp.approx.ftz.f64 %0, %1;" : "=d"( r ) : "d"( d ) );
-    const double e = fma( -d, r, 1.0 );
-    return fma( r, fma( e, e, e ), r );
-}
-
 // D <- -T^-1 for a symmetric positive definite 8 x 8 tile T held as an mma
 // accumulator (lane 4 g + t: c0, c1 = row g, columns 2t and 2t + 1), by sweeps on
 // the four 2 x 2 pivot blocks P (rows and columns p): A_pp -> -P^-1, A_rp -> A_rp

@@ -29,6 +29,7 @@
 #include "ipm_kernels.cuh"
 #include "kernels.h"
 #include "newton_batch.cuh"
+#include "small_cells.cuh"
 #include "uqc.h"
 
 using namespace uqc;
@@ -78,6 +79,7 @@ struct uqc_solver {
     int closureBlock = 256, closureGrid = 0, updateBlock = 256, updateGrid = 0, auxGrid = 0, auxBlock = 256;
     size_t closureSmem = 0, updateSmem = 0, initSmem = 0, mvSmem = 0, checkSmem = 0;
     int checkBlock = 256, checkGrid = 0;
+    void *checkFn = nullptr, *updateFn = nullptr;    // the check kernel, and the update kernel the steps launch
     int* d_activeList = nullptr;    // cells that need Newton: two lists (running step, next step)
     double* d_cellDt  = nullptr;    // per cell: CFL step of its nodal states
     double* d_uRe     = nullptr;    // moments re-projected by the closure epilogue (input of k_update)
@@ -270,6 +272,7 @@ KParams make_params( const uqc_solver* h ) {
     for( size_t i = 0; i < h->cfg.sigma.size() && i < 4; ++i ) ph.sigma[i] = h->cfg.sigma[i];
     ph.dimXi   = h->tab.dimXi;
     ph.dtFixed = h->area0 * h->cfg.cfl / 12.0;    // TimeSolver (timesolver.cpp:4-9)
+    ph.swSpeed = 0.5 / ( h->cfg.cfl / 12.0 );
     P.phi          = h->d_phi;
     P.phiWf        = h->d_phiWf;
     P.xi           = h->d_xi;
@@ -340,7 +343,14 @@ void* pick( int cl, int group, int which ) {
     return fn;
 }
 
-void* pick_check( int cl ) { return pick( cl, 32, KERNEL_CHECK ); }
+// A small-cell kernel, or null where the closure or the moment count has none.
+void* pick_small( int cl, int ntm, int which ) {
+    try {
+        return pick( cl, ntm, which );
+    } catch( const ConfigError& ) {
+        return nullptr;
+    }
+}
 
 int closure_np( int cl ) {
     const int ns = closure_states( cl );
@@ -655,6 +665,48 @@ void plan_newton( uqc_solver* h, int maxSmem ) {
     }
 }
 
+// The several-lanes-per-cell check and update kernels instead of the warp-per-
+// cell ones, where an instance holds the moments in a lane's registers. Update,
+// warp per cell / lanes (us): Burgers, 10 moments, 20k cells 43 / 25, 200k 336 / 121;
+// adaptive shallow water, 50k cells 55 / 29, 1M 1063 / 410 (check 1177 / 472);
+// 2-D Euler, 6 moments, 10k cells 36 / 32, 100k 266 / 138, 10 moments, 100k cells
+// 351 / 294 but 10k cells 46 / 52 (with 10 moments of four states a lane needs all
+// its registers and an SM holds eight warps: only where the mesh is large enough).
+void plan_small( uqc_solver* h ) {
+    const int cl = h->cfg.closure, nT = h->tab.nT;
+    if( h->d_bndNormal != nullptr || h->mesh.nFaces != ( h->nS == 4 ? 3 : 2 ) ) return;
+    if( h->nS == 4 && nT > SMALL_NT[0] && h->mesh.nCells < 20000 ) return;
+    for( int ntm : SMALL_NT ) {
+        if( nT > ntm ) continue;
+        const size_t table = size_t( h->tab.nQ ) * h->ld * sizeof( double );
+        if( 2 * table > 64 * 1024 ) return;
+        auto shape = [&]( void* fn, size_t smem, int warps, int& block, int& grid ) {
+            block = 32 * ( warps > 0 ? std::min( warps, 8 ) : 8 );
+            allow_dynamic_smem( fn );
+            int occ = 0;
+            CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, fn, block, smem ) );
+            const int cells = block / LPC;
+            grid            = std::min( std::max( 1, occ ) * h->numSMs, std::max( 1, ( h->mesh.nCells + cells - 1 ) / cells ) );
+        };
+        if( void* fn = pick_small( cl, ntm, update_test_on( h ) ? KERNEL_UPDATE_SMALL : KERNEL_UPDATE_SMALL_PLAIN ) ) {
+            h->updateFn   = fn;
+            h->updateSmem = table;
+            shape( fn, table, h->updateWarpsOpt, h->updateBlock, h->updateGrid );
+            if( h->updateGrid > h->blockPartialCap ) {
+                if( h->d_blockPartial ) cudaFree( h->d_blockPartial );
+                h->d_blockPartial  = dalloc<double>( size_t( h->updateGrid ) );
+                h->blockPartialCap = h->updateGrid;
+            }
+        }
+        if( void* fn = pick_small( cl, ntm, KERNEL_CHECK_SMALL ) ) {
+            h->checkFn   = fn;
+            h->checkSmem = 2 * table;
+            shape( fn, 2 * table, h->checkWarpsOpt, h->checkBlock, h->checkGrid );
+        }
+        return;
+    }
+}
+
 void plan_launches( uqc_solver* h ) {
     ++h->planGen;
     int dev;
@@ -694,6 +746,7 @@ void plan_launches( uqc_solver* h ) {
         void* kf             = pick( cl, h->group, update_kernel_id( h, true ) );
         void* kp             = pick( cl, h->group, update_kernel_id( h, false ) );
         void* ku             = update_test_on( h ) ? kf : kp;    // the variant the steps launch
+        h->updateFn          = ku;
         allow_dynamic_smem( kf );
         allow_dynamic_smem( kp );
         // warps per CTA: the option, else the count of 8, 4 or 2 that keeps the
@@ -744,11 +797,13 @@ void plan_launches( uqc_solver* h ) {
         if( warps < 1 ) throw ConfigError( "check workspace exceeds shared memory" );
         h->checkBlock = 32 * warps;
         h->checkSmem  = wsc * warps + ( h->tablesInSmem ? tables : 0 );
-        void* kk      = pick_check( cl );
+        void* kk      = pick( cl, 32, KERNEL_CHECK );
+        h->checkFn    = kk;
         allow_dynamic_smem( kk );
         CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kk, h->checkBlock, h->checkSmem ) );
         h->checkGrid = std::min( std::max( 1, occ ) * h->numSMs, std::max( 1, ( h->mesh.nCells + warps - 1 ) / warps ) );
     }
+    plan_small( h );
     plan_newton( h, maxSmem );
     plan_mixed( h, maxSmem );
     plan_rounds( h, maxSmem );
@@ -1090,7 +1145,7 @@ void enqueue_closure_phase( uqc_solver* h, KParams P ) {
     step_lists( h, P );
     if( h->cfg.newtonMode != 2 ) {
         void* args[] = {&P};
-        launch( h, pick_check( h->cfg.closure ), h->checkGrid, h->checkBlock, h->checkSmem, args );
+        launch( h, h->checkFn, h->checkGrid, h->checkBlock, h->checkSmem, args );
     }
     launch_closure( h, P, 1 );
 }
@@ -1099,8 +1154,7 @@ void enqueue_update( uqc_solver* h, KParams P ) {
     step_lists( h, P );
     P.finishInUpdate = update_test_on( h );
     void* args[]     = {&P};
-    launch( h, pick( h->cfg.closure, h->group, update_kernel_id( h, P.finishInUpdate != 0 ) ), h->updateGrid, h->updateBlock, h->updateSmem,
-            args );
+    launch( h, h->updateFn, h->updateGrid, h->updateBlock, h->updateSmem, args );
 }
 
 void enqueue_step( uqc_solver* h, KParams& P ) {
@@ -2190,7 +2244,7 @@ int uqc_step_host( uqc_solver* h, const double* u_in, const double* lambda_in, c
                     K.cellBase   = int( c0 );
                     K.nWork      = int( c1 - c0 );
                     void* args[] = {&K};
-                    CK( cudaLaunchKernel( pick_check( h->cfg.closure ), dim3( h->checkGrid ), dim3( h->checkBlock ), args, h->checkSmem,
+                    CK( cudaLaunchKernel( h->checkFn, dim3( h->checkGrid ), dim3( h->checkBlock ), args, h->checkSmem,
                                           h->checkStream ) );
                     ++h->launches;
                 }
@@ -2233,7 +2287,7 @@ int uqc_step_host( uqc_solver* h, const double* u_in, const double* lambda_in, c
             U.finishInUpdate = update_test_on( h );
             U.blockPartial   = h->d_chunkPartial;
             U.updChunks      = CHUNKS;
-            void* ku         = pick( h->cfg.closure, h->group, update_kernel_id( h, U.finishInUpdate != 0 ) );
+            void* ku         = h->updateFn;
             for( int c = 0; c < CHUNKS; ++c ) {
                 const size_t c0 = lo( c ), c1 = lo( c + 1 );
                 U.cellBase   = int( c0 );
