@@ -174,10 +174,10 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
  *                    kernel (default 16) and the mixed form's chord kernel
  *                    (default 16), each capped by shared memory; 0 = default.
  *   "closure_tiny"   systems of at most 6 duals per cell (states x moments)
- *                    on at most 64 nodes: -1 (default) / 1: the Newton of
- *                    each cell runs in registers on one warp (sums over nodes
- *                    by butterfly reduction, every lane solving the small
- *                    system itself), in both precisions (FP64 arithmetic);
+ *                    on at most 64 nodes: -1 (default) / 1: a kernel with the
+ *                    Newton of each cell on one warp (a lane per entry of the
+ *                    system, every lane solving it itself), in both
+ *                    precisions (FP64 arithmetic);
  *                    0: the general closure kernel.
  *   "closure_tables_smem"  1: the closure kernels stage the basis tables in
  *                    shared memory; 0: they read them through the L1 cache

@@ -22,7 +22,7 @@ enum KernelId {
     KERNEL_INVERT_SWEEP  = 12,   // k_invert_sweep (from k_hess_tc's values, n <= 84)
     KERNEL_UPDATE_WALL   = 13,   // k_update for meshes with wall cells (2-D Euler)
     KERNEL_UPDATE_PLAIN_WALL = 14,
-    KERNEL_CLOSURE_TINY      = 15,   // k_closure with the register Newton of tiny systems
+    KERNEL_CLOSURE_TINY      = 15,   // k_newton_tiny
     KERNEL_UPDATE_SPLIT      = 16,   // k_update (with / without the test) whose projection splits
     KERNEL_UPDATE_PLAIN_SPLIT = 17,  // the nodes of a small last block of basis functions
     KERNEL_NEWTON_S4          = 18,  // k_newton (2-D Euler): 4 cells on 4 warps, 4 CTAs per SM, at most 8 row tiles of pairs

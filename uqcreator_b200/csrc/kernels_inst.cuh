@@ -5,6 +5,7 @@
 #include "ipm_kernels.cuh"
 #include "kernels.h"
 #include "newton_batch.cuh"
+#include "newton_tiny.cuh"
 #include "small_cells.cuh"
 
 namespace uqc {
@@ -35,7 +36,7 @@ template <int CL> void* kernel_of( int group, int which ) {
             if( group == 256 ) return (void*)&k_closure<CL, 256, double>;
             return nullptr;
         case KERNEL_CLOSURE_TINY:
-            if constexpr( !Closure<CL>::LINEAR ) return (void*)&k_closure<CL, 32, double, true>;
+            if constexpr( !Closure<CL>::LINEAR ) return (void*)&k_newton_tiny<CL>;
             return nullptr;
         case KERNEL_CLOSURE_MIXED:
             if constexpr( !Closure<CL>::LINEAR ) {

@@ -394,12 +394,7 @@ __global__ void __launch_bounds__( 32 * W, CTAS ) k_newton( KParams P, int mode 
 #pragma unroll
                     for( int s = 0; s < NS; ++s ) L[s] = fma( li[s], r, L[s] );
                 }
-                if constexpr( CL == 1 )
-                    Closure<CL>::UDU( L, u, y, P.phys );
-                else {
-                    Closure<CL>::U( L, u, true, P.phys );
-                    Closure<CL>::DU( L, y, P.phys );
-                }
+                closure_udu<CL>( L, u, y, P.phys );
                 const double w = __ldg( P.wt + k );
 #pragma unroll
                 for( int s = 0; s < NS; ++s ) uk[k * NS + s] = u[s];

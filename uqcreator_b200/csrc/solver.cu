@@ -29,6 +29,7 @@
 #include "ipm_kernels.cuh"
 #include "kernels.h"
 #include "newton_batch.cuh"
+#include "newton_tiny.cuh"
 #include "small_cells.cuh"
 #include "uqc.h"
 
@@ -49,8 +50,10 @@ struct uqc_solver {
     int blockPartialCap = 0;           // doubles in d_blockPartial
     double* d_chunkPartial = nullptr;  // uqc_step_host's chunked update: a partial per CTA and launch
     int chunkPartialCap    = 0;
-    bool closureTiny = false;          // planned: the register Newton of tiny systems (k_closure TINY)
+    bool closureTiny = false;          // planned: the Newton of tiny systems (k_newton_tiny)
     int tinyGrid     = 0;
+    size_t tinySmem  = 0;
+    double* d_tinyTab = nullptr;
     // FP64 closure of large systems: k_newton's instance (a KernelId, 0: k_closure) and launch shape
     int newtonId = 0, newtonBlock = 0, newtonGrid = 0;
     // UQC_MIXED runs k_newton (FP64) where it is faster than the mixed kernels: in
@@ -281,6 +284,7 @@ KParams make_params( const uqc_solver* h ) {
     P.phiT         = h->d_phiT;
     P.ldT          = ( h->tab.nQ + 3 ) & ~3;
     P.pairSlots    = h->d_pairSlots;
+    P.tinyTab      = h->d_tinyTab;
     P.tabInSmem    = h->newtonTab ? 1 : 0;
     P.tablesInSmem = h->tablesInSmem;
     P.area         = h->d_area;
@@ -731,13 +735,22 @@ void plan_launches( uqc_solver* h ) {
     int occ = 0;
     CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kc, h->closureBlock, h->closureSmem ) );
     h->closureGrid = std::max( 1, occ ) * h->numSMs;
-    // tiny systems (n <= TINY_N duals, <= 64 nodes): the register Newton, a warp per cell
-    h->closureTiny = h->tinyOpt != 0 && h->closureGroup == 32 && n <= size_t( TINY_N ) && nQ <= 64 && !closure_linear( cl );
+    // tiny systems (n <= TINY_N duals, at most 64 nodes): k_newton_tiny, a warp per cell
+    h->closureTiny =
+        h->tinyOpt != 0 && h->closureGroup == 32 && n <= size_t( TINY_N ) && nQ <= TINY_MAX_NODES && !closure_linear( cl );
     if( h->closureTiny ) {
-        void* kt = pick( cl, 32, KERNEL_CLOSURE_TINY );
+        void* kt    = pick( cl, 32, KERNEL_CLOSURE_TINY );
+        h->tinySmem = ( size_t( 32 ) * nQ + 4 * size_t( tiny_warp_doubles( nS, closure_np( cl ), nQ ) ) ) * sizeof( double );
         allow_dynamic_smem( kt );
-        CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kt, h->closureBlock, h->closureSmem ) );
+        CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kt, 128, h->tinySmem ) );
         h->tinyGrid = std::max( 1, occ ) * h->numSMs;
+        if( !h->d_tinyTab ) {
+            std::vector<double> tab( size_t( 32 ) * nQ );
+            for( int k = 0; k < nQ; ++k )
+                for( int e = 0; e < 32; ++e )
+                    tab[size_t( 32 ) * k + e] = tiny_entry( nS, nT, &h->tab.phi[size_t( k ) * nT], h->padWt[k], e );
+            h->d_tinyTab = dupload( tab );
+        }
     }
     // update kernel: a warp per cell; phiWf + one node-flux buffer per warp
     {
@@ -1024,7 +1037,7 @@ void release( uqc_solver* h ) {
                     (void*)h->d_unitN, (void*)h->d_scaledN, (void*)h->d_nbr, (void*)h->d_boundary, (void*)h->d_u, (void*)h->d_lam,
                     (void*)h->d_bndNormal, (void*)h->d_uQ, (void*)h->d_uOld0, (void*)h->d_blockPartial, (void*)h->d_chunkPartial, (void*)h->d_level, (void*)h->d_status,
                     (void*)h->d_iters, (void*)h->d_ctl, (void*)h->d_xLam, (void*)h->d_xU, (void*)h->d_xNt, (void*)h->d_xStatus,
-                    (void*)h->d_xIters, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_phiT, (void*)h->d_pairSlots, (void*)h->d_fallbackList,
+                    (void*)h->d_xIters, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_phiT, (void*)h->d_pairSlots, (void*)h->d_tinyTab, (void*)h->d_fallbackList,
                     (void*)h->d_factorStore, (void*)h->d_factorLevel, (void*)h->d_gStore, (void*)h->d_v2Lists,
                     (void*)h->d_chordIters, (void*)h->d_qTiles, (void*)h->d_sendCells, (void*)h->d_filter, (void*)h->d_lassoParam,
                     (void*)h->d_lassoL1} )
@@ -1064,10 +1077,8 @@ void launch_closure( uqc_solver* h, KParams& P, int mode ) {
     if( h->closureTiny && h->cfg.newtonMode != 2 ) {
         // tiny systems: the FP64 register Newton in both precisions (the mixed
         // form's FP32 Hessian saves nothing at this size)
-        KParams Q      = P;
-        Q.tablesInSmem = h->closureTablesInSmem;
-        void* args[]   = {&Q, &mode};
-        launch( h, pick( h->cfg.closure, 32, KERNEL_CLOSURE_TINY ), h->tinyGrid, h->closureBlock, h->closureSmem, args );
+        void* args[] = {&P, &mode};
+        launch( h, pick( h->cfg.closure, 32, KERNEL_CLOSURE_TINY ), h->tinyGrid, 128, h->tinySmem, args );
         return;
     }
     if( mode == 1 && P.gStore ) {
