@@ -78,6 +78,7 @@ struct uqc_solver {
     unsigned* d_xNt = nullptr;
     int *d_xStatus = nullptr, *d_xIters = nullptr;
     size_t xCap = 0;
+    void* h_batch = nullptr;    // uqc_closure_solve_host: pinned memory of a few cells' batch (HOST_BATCH_BYTES)
     // launch shapes
     int closureBlock = 256, closureGrid = 0, updateBlock = 256, updateGrid = 0, auxGrid = 0, auxBlock = 256;
     size_t closureSmem = 0, updateSmem = 0, initSmem = 0, mvSmem = 0, checkSmem = 0;
@@ -1043,6 +1044,7 @@ void release( uqc_solver* h ) {
                     (void*)h->d_lassoL1} )
         if( p ) cudaFree( p );
     if( h->h_ctl ) cudaFreeHost( h->h_ctl );
+    if( h->h_batch ) cudaFreeHost( h->h_batch );
     for( auto& e : h->ev )
         if( e ) cudaEventDestroy( e );
     if( h->asyncEv ) cudaEventDestroy( h->asyncEv );
@@ -2411,46 +2413,84 @@ static void closure_on( uqc_solver* h, int n, double* d_lam, const double* d_u, 
     CK( cudaGetLastError() );
 }
 
+// Batches up to this size are read and written over PCIe by the kernel itself:
+// below it the copies' fixed cost is the larger one.
+static constexpr size_t HOST_BATCH_BYTES = 16 * 1024;
+
 int uqc_closure_solve_host( uqc_solver* h, int n, double* lambda, const double* u, const unsigned* n_total, int layout, int* status ) {
     if( !h || n < 0 || !lambda || !u || ( layout != UQC_LAYOUT_REF && layout != UQC_LAYOUT_STATE_MAJOR ) ) return UQC_ERR_ARGUMENT;
     if( n == 0 ) return UQC_OK;
     return guarded_dev( h, [&] {
         h->launches = 0;
-        ensure_scratch( h, size_t( n ) );
         const size_t cnt = size_t( n ) * h->ldc, nT = size_t( h->tab.nT ), nS = size_t( h->nS );
-        std::vector<double> L( cnt ), U( cnt );
-        for( size_t j = 0; j < size_t( n ); ++j )
-            for( size_t s = 0; s < nS; ++s )
-                for( size_t i = 0; i < nT; ++i ) {
-                    size_t sm = j * nS * nT + s * nT + i, src = layout == UQC_LAYOUT_REF ? j * nS * nT + i * nS + s : sm;
-                    L[sm] = lambda[src];
-                    U[sm] = u[src];
-                }
-        std::vector<unsigned> nt( n, unsigned( nT ) );
         if( n_total )
-            for( int j = 0; j < n; ++j ) {
+            for( int j = 0; j < n; ++j )
                 if( std::find( h->tab.nTLevel.begin(), h->tab.nTLevel.end(), int( n_total[j] ) ) == h->tab.nTLevel.end() )
                     throw std::invalid_argument( "n_total[" + std::to_string( j ) + "] is not a refinement level size" );
-                nt[j] = n_total[j];
+        // state-major cells in dst from the caller's layout, and back
+        auto gather = [&]( double* dst, const double* src ) {
+            if( layout == UQC_LAYOUT_STATE_MAJOR ) {
+                std::memcpy( dst, src, cnt * sizeof( double ) );
+                return;
             }
-        CK( cudaMemcpyAsync( h->d_xLam, L.data(), cnt * sizeof( double ), cudaMemcpyHostToDevice, h->stream ) );
-        CK( cudaMemcpyAsync( h->d_xU, U.data(), cnt * sizeof( double ), cudaMemcpyHostToDevice, h->stream ) );
-        CK( cudaMemcpyAsync( h->d_xNt, nt.data(), n * sizeof( unsigned ), cudaMemcpyHostToDevice, h->stream ) );
-        closure_on( h, n, h->d_xLam, h->d_xU, h->d_xNt, h->d_xStatus, h->d_xIters );
-        std::vector<int> st( n );
-        CK( cudaMemcpyAsync( L.data(), h->d_xLam, cnt * sizeof( double ), cudaMemcpyDeviceToHost, h->stream ) );
-        CK( cudaMemcpyAsync( st.data(), h->d_xStatus, n * sizeof( int ), cudaMemcpyDeviceToHost, h->stream ) );
-        CK( cudaStreamSynchronize( h->stream ) );
-        for( size_t j = 0; j < size_t( n ); ++j )
-            for( size_t s = 0; s < nS; ++s )
-                for( size_t i = 0; i < nT; ++i ) {
-                    size_t sm = j * nS * nT + s * nT + i, dst = layout == UQC_LAYOUT_REF ? j * nS * nT + i * nS + s : sm;
-                    lambda[dst] = L[sm];
+            for( size_t j = 0; j < size_t( n ); ++j )
+                for( size_t s = 0; s < nS; ++s )
+                    for( size_t i = 0; i < nT; ++i ) dst[j * nS * nT + s * nT + i] = src[j * nS * nT + i * nS + s];
+        };
+        auto scatter = [&]( double* dst, const double* src ) {
+            if( layout == UQC_LAYOUT_STATE_MAJOR ) {
+                std::memcpy( dst, src, cnt * sizeof( double ) );
+                return;
+            }
+            for( size_t j = 0; j < size_t( n ); ++j )
+                for( size_t s = 0; s < nS; ++s )
+                    for( size_t i = 0; i < nT; ++i ) dst[j * nS * nT + i * nS + s] = src[j * nS * nT + s * nT + i];
+        };
+        std::vector<int> st;
+        const int* stat = nullptr;
+        if( 2 * cnt * sizeof( double ) + 3 * size_t( n ) * sizeof( int ) <= HOST_BATCH_BYTES ) {
+            // a few cells: the kernel works on pinned host memory, one launch and no copies
+            if( !h->h_batch ) CK( cudaMallocHost( &h->h_batch, HOST_BATCH_BYTES ) );
+            double* L    = reinterpret_cast<double*>( h->h_batch );
+            double* U    = L + cnt;
+            unsigned* nt = reinterpret_cast<unsigned*>( U + cnt );
+            int* s       = reinterpret_cast<int*>( nt + n );
+            gather( L, lambda );
+            gather( U, u );
+            if( n_total ) std::memcpy( nt, n_total, size_t( n ) * sizeof( unsigned ) );
+            closure_on( h, n, L, U, n_total ? nt : nullptr, s, s + n );
+            CK( cudaStreamSynchronize( h->stream ) );
+            scatter( lambda, L );
+            stat = s;
+        }
+        else {
+            ensure_scratch( h, size_t( n ) );
+            std::vector<double> L;
+            if( layout == UQC_LAYOUT_REF ) L.resize( cnt );
+            auto upload = [&]( double* d, const double* src ) {
+                if( layout == UQC_LAYOUT_REF ) {
+                    gather( L.data(), src );
+                    src = L.data();
                 }
+                CK( cudaMemcpyAsync( d, src, cnt * sizeof( double ), cudaMemcpyHostToDevice, h->stream ) );
+                if( layout == UQC_LAYOUT_REF ) CK( cudaStreamSynchronize( h->stream ) );    // L is used again
+            };
+            upload( h->d_xU, u );
+            upload( h->d_xLam, lambda );
+            if( n_total ) CK( cudaMemcpyAsync( h->d_xNt, n_total, size_t( n ) * sizeof( unsigned ), cudaMemcpyHostToDevice, h->stream ) );
+            closure_on( h, n, h->d_xLam, h->d_xU, n_total ? h->d_xNt : nullptr, h->d_xStatus, h->d_xIters );
+            st.resize( n );
+            double* out = layout == UQC_LAYOUT_REF ? L.data() : lambda;
+            CK( cudaMemcpyAsync( out, h->d_xLam, cnt * sizeof( double ), cudaMemcpyDeviceToHost, h->stream ) );
+            CK( cudaMemcpyAsync( st.data(), h->d_xStatus, n * sizeof( int ), cudaMemcpyDeviceToHost, h->stream ) );
+            CK( cudaStreamSynchronize( h->stream ) );
+            if( layout == UQC_LAYOUT_REF ) scatter( lambda, L.data() );
+            stat = st.data();
+        }
         int bad = 0;
         for( int j = 0; j < n; ++j ) {
-            if( status ) status[j] = st[j];
-            bad += st[j] != 0;
+            if( status ) status[j] = stat[j];
+            bad += stat[j] != 0;
         }
         return bad ? fail( h, UQC_ERR_NOT_CONVERGED, std::to_string( bad ) + " cells did not converge" ) : UQC_OK;
     } );
@@ -2462,14 +2502,7 @@ int uqc_closure_solve_device( uqc_solver* h, int n, double* d_lambda, const doub
     return guarded_dev( h, [&] {
         h->launches = 0;
         ensure_scratch( h, size_t( n ) );
-        unsigned* nt = const_cast<unsigned*>( d_n_total );
-        if( !nt ) {
-            std::vector<unsigned> v( n, unsigned( h->tab.nT ) );
-            CK( cudaMemcpyAsync( h->d_xNt, v.data(), n * sizeof( unsigned ), cudaMemcpyHostToDevice, h->stream ) );
-            CK( cudaStreamSynchronize( h->stream ) );
-            nt = h->d_xNt;
-        }
-        closure_on( h, n, d_lambda, d_u, nt, d_status ? d_status : h->d_xStatus, h->d_xIters );
+        closure_on( h, n, d_lambda, d_u, d_n_total, d_status ? d_status : h->d_xStatus, h->d_xIters );
         return UQC_OK;
     } );
 }
