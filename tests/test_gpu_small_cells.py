@@ -1,7 +1,7 @@
-"""The check and update kernels of cells with few moments: several lanes per
-cell, instances of 6, 10 and 16 moments; cell counts that leave a warp partly
-empty, node counts that leave lanes idle, with and without the next step's
-test, against the FP64 oracle."""
+"""The check and update kernels of cells with few moments (several lanes per
+cell; instances of 6, 10 and 16 moments) and the 2-D Euler update on the tensor
+cores: cell counts that leave a warp partly empty, node counts that leave lanes
+idle, with and without the next step's test, against the FP64 oracle."""
 import numpy as np
 import pytest
 
@@ -22,6 +22,13 @@ CASES = {
     "sw_16_moments": W.shallow_water1d(ncells=70, max_degree=15, nquad=32, tend=10.0),
     "euler_3_moments": W.euler2d(nx=7, ny=3, degree=1, nquad=3, tend=10.0),
     "euler_6_moments": W.euler2d(nx=16, ny=5, degree=2, nquad=5, tend=10.0),
+    # k_update_mma: two cells a warp (odd counts of cells per warp and mesh), its three
+    # widths, node counts that are not multiples of 4, the table in chunks
+    "euler_10_moments": W.euler2d(nx=9, ny=5, degree=3, nquad=5, tend=10.0),
+    "euler_15_moments": W.euler2d(nx=11, ny=3, degree=4, nquad=7, tend=10.0),
+    "euler_28_moments": W.euler2d(nx=7, ny=4, degree=6, nquad=9, tend=10.0),
+    "euler_45_moments": W.euler2d(nx=6, ny=3, degree=8, nquad=10, tend=10.0),
+    "euler_35_moments_chunks": W.euler2d(nx=6, ny=4, degree=4, nquad=7, dim_xi=3, tend=10.0),
 }
 
 
@@ -43,18 +50,3 @@ def test_steps_match_oracle(name, update_test):
     uo, _, vo = o.get_state()
     np.testing.assert_array_equal(vs, vo)
     np.testing.assert_allclose(us, uo, rtol=0, atol=1e-9 * np.abs(uo).max())
-
-
-def test_large_mesh_of_ten_moments():
-    """2-D Euler with 10 moments takes these kernels only from 20,000 cells on:
-    its two instances (option update_test) against each other."""
-    toml = W.euler2d(nx=120, ny=90, degree=3, nquad=6, tend=10.0)
-    out = []
-    for v in (0, 1):
-        s = Solver(toml)
-        s.set_option("update_test", v)
-        s.init_state()
-        s.step(3)
-        out.append(s.download_state()[0])
-        s.close()
-    np.testing.assert_allclose(out[0], out[1], rtol=0, atol=1e-9 * np.abs(out[0]).max())

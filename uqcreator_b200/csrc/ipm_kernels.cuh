@@ -112,6 +112,9 @@ struct KParams {
     const double* phiT;      // nT x ldT: phi node-contiguous, zero from nQ to ldT (k_newton)
     int ldT;                 // nQ rounded up to 4
     const double* tinyTab;   // k_newton_tiny: nQ x 32, column e the table of its sum e
+    const double* phiWfP;    // k_update_mma: phiWf padded with zeros, nQ rounded up to 4 rows of ldP
+    int ldP;
+    int updNodes;            // k_update_mma: nodes per chunk (a multiple of 4; all of them: the table stays)
     int tabInSmem;           // k_newton: phiT staged in shared memory
     const unsigned* pairSlots;    // k_newton: places of each (pair, block) in the Hessian tiles (low and high half)
     bool tablesInSmem;
@@ -317,15 +320,19 @@ template <int NS, int GROUP>
 __device__ __forceinline__ double gradient_sums( const Grp<GROUP>& g, const KParams& P, const double* phiWf, const double* uk, const double* uh,
                                                  int nTj, double* gout, double* ms ) {
     double sq = 0.0;
+    int whole = nTj;    // basis functions [0, whole) take a lane each over all nodes
     if constexpr( GROUP == 32 ) {
-        if( nTj <= 16 ) {
-            // few basis functions: the warp splits the nodes as well, lane =
-            // i + w part (w = nTj rounded up to a power of two), each part
-            // summing the nodes k = part (mod 32 / w), then a butterfly over
-            // the parts (a fixed order, so the sums are reproducible)
+        // what is left beyond blocks of 32, when it is at most 16 functions (all of
+        // them, or a last block), splits the nodes as well: lane = i + w part (w =
+        // their number rounded up to a power of two), each part summing the nodes
+        // k = part (mod 32 / w), then a butterfly over the parts (a fixed order, so
+        // the sums are reproducible)
+        const int m = nTj & 31;
+        if( m > 0 && m <= 16 ) {
+            whole = nTj - m;
             int w = 1;
-            while( w < nTj ) w <<= 1;
-            const int i = g.r & ( w - 1 ), part = g.r / w, parts = 32 / w;
+            while( w < m ) w <<= 1;
+            const int i = whole + ( g.r & ( w - 1 ) ), part = g.r / w, parts = 32 / w;
             double a[NS];
 #pragma unroll
             for( int st = 0; st < NS; ++st ) a[st] = 0.0;
@@ -349,11 +356,11 @@ __device__ __forceinline__ double gradient_sums( const Grp<GROUP>& g, const KPar
                     sq += d * d;
                 }
             }
-            return sq;
+            if( whole == 0 ) return sq;
         }
     }
     if constexpr( GROUP <= 64 ) {
-        for( int i = g.r; i < nTj; i += GROUP ) {
+        for( int i = g.r; i < whole; i += GROUP ) {
             double a[NS];
 #pragma unroll
             for( int s = 0; s < NS; ++s ) a[s] = 0.0;
@@ -1110,12 +1117,10 @@ template <int CL> __global__ void __launch_bounds__( 512, 2 ) k_check( KParams P
             CT_BEGIN( tlu );
             // U(Lambda_k) at every node, Lambda_k in registers (closure.cpp:205-213, 234-253)
             for( int k = g.r; k < P.nQ; k += 32 ) {
-                const double* row = phi + size_t( k ) * P.ld;
                 double Lk[NS], y[NS];
 #pragma unroll
                 for( int s = 0; s < NS; ++s ) Lk[s] = 0.0;
-                for( int i = 0; i < nTj; ++i ) {
-                    const double r = row[i];
+                auto add = [&]( int i, double r ) {
                     double li[NS];
                     if constexpr( Closure<CL>::LINEAR ) {
 #pragma unroll
@@ -1135,6 +1140,16 @@ template <int CL> __global__ void __launch_bounds__( 512, 2 ) k_check( KParams P
                     }
 #pragma unroll
                     for( int s = 0; s < NS; ++s ) Lk[s] = fma( li[s], r, Lk[s] );
+                };
+                if( P.tablesInSmem ) {
+                    const double* row = phi + size_t( k ) * P.ld;
+                    for( int i = 0; i < nTj; ++i ) add( i, row[i] );
+                }
+                else {
+                    // the table in memory node-contiguous: a warp's nodes in whole lines
+                    // (by rows each value of a warp's nodes is a line of its own)
+                    const double* col = P.phiT + k;
+                    for( int i = 0; i < nTj; ++i, col += P.ldT ) add( i, __ldg( col ) );
                 }
                 Closure<CL>::U( Lk, y, true, P.phys );
 #pragma unroll
@@ -1271,6 +1286,65 @@ __device__ __forceinline__ void finish_cell( const KParams& P, int cell, double 
     dtNext         = d < dtNext ? d : dtNext;
 }
 
+// The next step's lists of an update kernel (a warp's cells).
+struct NextLists {
+    int *nlist = nullptr, *clist = nullptr;              // Newton list, check list
+    unsigned *ncount = nullptr, *ccount = nullptr;
+    WarpListBuf nbuf, cbuf;
+    __device__ __forceinline__ void open( const KParams& P ) {
+        step_list( P, 1, nlist, ncount );
+        clist  = P.checkList + size_t( ( P.ctl->steps + 1 ) & 1 ) * P.nCells;
+        ccount = P.checkCount + ( ( P.ctl->steps + 1 ) & 1 );
+    }
+    __device__ __forceinline__ void flush( int lane ) {
+        nbuf.flush( lane, nlist, ncount );
+        cbuf.flush( lane, clist, ccount );
+    }
+};
+
+// The next step's closure test of a cell by the warp that updated it. sq: ||u_re -
+// u_new||^2, the same in every lane; u00: u_new(0, 0) (lane 0's).
+template <int NS>
+__device__ __forceinline__ void test_next_step( const KParams& P, int lane, int cell, int nTj, double sq, double u00, NextLists& N,
+                                                double& dtNext ) {
+    const size_t ldc = size_t( NS ) * P.nT;
+    // The next step's closure test, here: its gradient is
+    // sum_k U(Lambda_k) phiWf(k, i) - u_new = uRe - u_new, because uRe was
+    // re-projected from the same duals' nodal states (which this kernel
+    // just used). A cell that passes (and keeps its level) would only
+    // be re-projected onto uRe again: it skips the closure and keeps
+    // uRe; the others go to the next step's list.
+    const bool pass = sqrt( sq ) < P.eps;
+    bool fin        = pass;
+    if( fin && P.nLevels > 1 ) {
+        // the level rule of the epilogue, on u_new(0, .) in the same order
+        __syncwarp();    // the cell's new moments are written
+        const int lev   = int( P.level[cell] );
+        const double* u = P.u + cell * ldc;
+        auto at         = [&]( int i ) { return u[i]; };
+        if( level_rule( P, level_indicator( P, at, lev, nTj ), lev ) != lev ) fin = false;
+    }
+    if( fin ) {
+        if( lane == 0 ) finish_cell( P, cell, u00, dtNext );
+    }
+    else if( pass )
+        N.cbuf.push( lane, cell, N.clist, N.ccount );    // converged, new level: k_check's epilogue
+    else {
+        if( P.gStore ) {
+            // the gradient the mixed form's Newton starts from: uRe - u_new,
+            // the same differences as gi above (from the values just stored)
+            __syncwarp();
+            double* gs = P.gStore + size_t( cell ) * P.gStride;
+            for( int idx = lane; idx < NS * nTj; idx += 32 ) {
+                const int s = idx / nTj, i = idx - s * nTj;
+                gs[idx]     = P.uRe[cell * ldc + s * P.nT + i] - P.u[cell * ldc + s * P.nT + i];
+            }
+            if( lane == 0 ) gs[ldc] = sqrt( sq );
+        }
+        N.nbuf.push( lane, cell, N.nlist, N.ncount );
+    }
+}
+
 // End of an update kernel, by every CTA: the CTA's part of the residual (res per
 // thread), and in the last CTA to arrive the residual of the step and the loop
 // control. The sums have a fixed order: per thread, warp and CTA, then over the
@@ -1379,16 +1453,8 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
     const size_t ldc = size_t( NS ) * P.nT;
     double res       = 0.0;
     double dtNext    = 1e300;    // lane 0: min dt of the cells finished for the next step
-    int* nlist       = nullptr;
-    unsigned* ncount = nullptr;
-    if( finish ) step_list( P, 1, nlist, ncount );
-    int* clist        = nullptr;
-    unsigned* ccount  = nullptr;
-    if( finish ) {
-        clist  = P.checkList + size_t( ( P.ctl->steps + 1 ) & 1 ) * P.nCells;
-        ccount = P.checkCount + ( ( P.ctl->steps + 1 ) & 1 );
-    }
-    WarpListBuf nbuf, cbuf;    // next step's active list and check list
+    NextLists N;
+    if( finish ) N.open( P );
     for( int cell = P.cellBase + blockIdx.x * nWarps + warp; cell < P.cellBase + P.nWork; cell += gridDim.x * nWarps ) {
         const int bc = P.boundary[cell];
         if( finish && lane == 0 && P.finFlag[cell] ) {
@@ -1407,7 +1473,7 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
                 if( finish && P.nLevels == 1 ) finish_cell( P, cell, u0, dtNext );
             }
             // with refinement levels k_check's epilogue applies the level rule
-            if( finish && P.nLevels > 1 ) cbuf.push( lane, cell, clist, ccount );
+            if( finish && P.nLevels > 1 ) N.cbuf.push( lane, cell, N.clist, N.ccount );
             continue;
         }
         const int nTj    = P.nTLevel[P.level[cell]];
@@ -1563,7 +1629,7 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
         // independent chains sharing each table value
         const double c = dt / P.area[cell];
         double sq      = 0.0;
-        double v0a = 0.0, v0b = 0.0;    // u_new(0, lane) and u_new(0, lane + 32), for the level rule
+        double v00     = 0.0;    // u_new(0, 0), lane 0
         auto apply     = [&]( int i, const double* old, const double* r ) {
 #pragma unroll
             for( int s = 0; s < NS; ++s ) {
@@ -1571,9 +1637,10 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
                 const double gi  = old[s] - v;
                 P.u[cell * ldc + s * P.nT + i] = v;
                 sq                             = fma( gi, gi, sq );
-                if( s == 0 && i < 32 ) v0a = v;
-                if( s == 0 && i >= 32 && i < 64 ) v0b = v;
-                if( s == 0 && i == 0 ) res += fabs( v - P.uOld0[cell] ) * P.area[cell];
+                if( s == 0 && i == 0 ) {
+                    v00 = v;
+                    res += fabs( v - P.uOld0[cell] ) * P.area[cell];
+                }
             }
         };
         if constexpr( !SPLIT ) {
@@ -1618,58 +1685,29 @@ __global__ void __launch_bounds__( 256, ( update_min_ctas<CL, FIN>() ) ) k_updat
             }
         }
         if( finish ) {
-            // The next step's closure test, here: its gradient is
-            // sum_k U(Lambda_k) phiWf(k, i) - u_new = uRe - u_new, because uRe was
-            // re-projected from the same duals' nodal states (which this kernel
-            // just used). A cell that passes (and keeps its level) would only
-            // be re-projected onto uRe again: it skips the closure and keeps
-            // uRe; the others go to the next step's list.
             for( int o = 16; o > 0; o >>= 1 ) sq += __shfl_xor_sync( 0xffffffffu, sq, o );
-            sq              = __shfl_sync( 0xffffffffu, sq, 0 );    // one decision for the warp
-            const bool pass = sqrt( sq ) < P.eps;
-            bool fin        = pass;
-            if( fin && P.nLevels > 1 ) {
-                // the level rule of the epilogue, on u_new(0, .) in the same order
-                // (values from the lanes' registers; beyond 64 moments from memory)
-                __syncwarp();
-                const int lev = int( P.level[cell] );
-                auto at       = [&]( int i ) {
-                    const double r = __shfl_sync( 0xffffffffu, ( i >> 5 ) ? v0b : v0a, i & 31 );
-                    return i < 64 ? r : P.u[cell * ldc + i];
-                };
-                if( level_rule( P, level_indicator( P, at, lev, nTj ), lev ) != lev ) fin = false;
-            }
-            if( fin ) {
-                if( lane == 0 ) finish_cell( P, cell, v0a, dtNext );
-            }
-            else if( pass )
-                cbuf.push( lane, cell, clist, ccount );    // converged, new level: k_check's epilogue
-            else {
-                if( P.gStore ) {
-                    // the gradient the mixed form's Newton starts from: uRe - u_new,
-                    // the same differences as gi above (from the values just stored)
-                    __syncwarp();
-                    double* gs = P.gStore + size_t( cell ) * P.gStride;
-                    for( int idx = lane; idx < NS * nTj; idx += 32 ) {
-                        const int s = idx / nTj, i = idx - s * nTj;
-                        gs[idx]     = P.uRe[cell * ldc + s * P.nT + i] - P.u[cell * ldc + s * P.nT + i];
-                    }
-                    if( lane == 0 ) gs[ldc] = sqrt( sq );
-                }
-                nbuf.push( lane, cell, nlist, ncount );
-            }
+            sq = __shfl_sync( 0xffffffffu, sq, 0 );    // one decision for the warp
+            test_next_step<NS>( P, lane, cell, nTj, sq, v00, N, dtNext );
         }
         __syncwarp();
     }
-    if( finish ) {
-        nbuf.flush( lane, nlist, ncount );
-        cbuf.flush( lane, clist, ccount );
-    }
+    if( finish ) N.flush( lane );
     if( lane == 0 && dtNext < 1e300 ) atomic_min_pos_double( &P.ctl->dtBitsNext, dtNext );
     update_epilogue( P, res, dt, finish );
 }
 
+// doubles per thread group of k_init's shared memory: nodal states (node-major),
+// the parts' sums
+__host__ __device__ inline size_t init_group_doubles( int nS, int nT, int nQ, int group ) {
+    const int parts = group / nT > 0 ? group / nT : 1;
+    return ( ( size_t( nS ) * nQ + size_t( parts ) * nS * nT ) + 3 ) & ~size_t( 3 );
+}
+
 // Initial moments u_j = U_IC(x_j, xi_k) phiWf and duals lambda_j(:,0) = DS(u_j(:,0)).
+// A thread per (part of the nodes, basis function) sums all states, as many
+// parts as the group holds, then the parts are added in order: with a thread per
+// moment over all nodes the longest sum set the time (262k cells of 140 moments,
+// 512 nodes: 12.8 ms).
 // keepMoments: the moments are already in place (restart without duals,
 // momentsolver.cpp:463-485); only the duals are set.
 template <int CL, int GROUP> __global__ void __launch_bounds__( GROUP == 32 ? 256 : GROUP ) k_init( KParams P, int keepMoments ) {
@@ -1677,23 +1715,41 @@ template <int CL, int GROUP> __global__ void __launch_bounds__( GROUP == 32 ? 25
     extern __shared__ __align__( 16 ) double smem[];
     const int groups = blockDim.x / GROUP;
     Grp<GROUP> g{int( threadIdx.x % GROUP ), 1 + int( threadIdx.x / GROUP )};
-    const int gid   = threadIdx.x / GROUP;
-    double* uic     = smem + size_t( gid ) * ( size_t( NS ) * P.nQ + 8 );
+    const int gid    = threadIdx.x / GROUP;
+    double* uic      = smem + size_t( gid ) * init_group_doubles( NS, P.nT, P.nQ, GROUP );
+    double* part     = uic + size_t( NS ) * P.nQ;
     const size_t ldc = size_t( NS ) * P.nT;
+    const int parts  = GROUP / P.nT > 0 ? GROUP / P.nT : 1;
     for( int cell = blockIdx.x * groups + gid; cell < P.nCells; cell += gridDim.x * groups ) {
-        for( int k = g.r; k < P.nQ && !keepMoments; k += GROUP ) {
-            double y[NS];
-            Problem<CL>::ic( P.center + 2 * cell, P.xi + size_t( k ) * P.dimXi, y, P.phys );
+        if( !keepMoments ) {
+            for( int k = g.r; k < P.nQ; k += GROUP ) {
+                double y[NS];
+                Problem<CL>::ic( P.center + 2 * cell, P.xi + size_t( k ) * P.dimXi, y, P.phys );
 #pragma unroll
-            for( int s = 0; s < NS; ++s ) uic[s * P.nQ + k] = y[s];
+                for( int s = 0; s < NS; ++s ) uic[k * NS + s] = y[s];
+            }
+            g.sync();
+            for( int e = g.r; e < parts * P.nT; e += GROUP ) {
+                const int p = e / P.nT, i = e - p * P.nT;
+                double a[NS];
+#pragma unroll
+                for( int s = 0; s < NS; ++s ) a[s] = 0.0;
+#pragma unroll 4
+                for( int k = p; k < P.nQ; k += parts ) {
+                    const double w = __ldg( P.phiWf + size_t( k ) * P.ld + i );
+#pragma unroll
+                    for( int s = 0; s < NS; ++s ) a[s] = fma( uic[k * NS + s], w, a[s] );
+                }
+#pragma unroll
+                for( int s = 0; s < NS; ++s ) part[( p * NS + s ) * P.nT + i] = a[s];
+            }
+            g.sync();
         }
-        g.sync();
         for( int idx = g.r; idx < int( ldc ); idx += GROUP ) {
-            int s = idx / P.nT, i = idx - s * P.nT;
             if( !keepMoments ) {
-                double a = 0.0;
-                for( int k = 0; k < P.nQ; ++k ) a = fma( uic[s * P.nQ + k], P.phiWf[size_t( k ) * P.ld + i], a );
-                P.u[cell * ldc + idx] = a;
+                double m = part[idx];
+                for( int p = 1; p < parts; ++p ) m += part[p * ldc + idx];
+                P.u[cell * ldc + idx] = m;
             }
             P.lam[cell * ldc + idx] = 0.0;
         }

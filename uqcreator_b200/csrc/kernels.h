@@ -31,7 +31,9 @@ enum KernelId {
     KERNEL_NEWTON_L2          = 21,  // ... 2 cells on 16 warps, at most 80
     KERNEL_CHECK_SMALL        = 22,  // k_check_small (group: its NTM), nonlinear closures
     KERNEL_UPDATE_SMALL       = 23,  // k_update_small with / without the next step's test (group: NTM)
-    KERNEL_UPDATE_SMALL_PLAIN = 24
+    KERNEL_UPDATE_SMALL_PLAIN = 24,
+    KERNEL_UPDATE_MMA         = 25,  // k_update_mma (2-D Euler) with / without the next step's test
+    KERNEL_UPDATE_MMA_PLAIN   = 26   // (group: its column tiles)
 };
 
 // nullptr when there is no such variant

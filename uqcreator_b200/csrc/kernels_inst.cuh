@@ -7,13 +7,14 @@
 #include "newton_batch.cuh"
 #include "newton_tiny.cuh"
 #include "small_cells.cuh"
+#include "update_mma.cuh"
 
 namespace uqc {
 
 // The instances for few moments: NTM = 6, 10 or 16, as far as a lane's registers
 // hold a cell's sums.
 template <int CL, int NTM> void* small_kernel_of( int which ) {
-    if constexpr( Closure<CL>::NS * NTM <= 40 ) {
+    if constexpr( Closure<CL>::NS * NTM <= ( Closure<CL>::NS == 4 ? 24 : 32 ) ) {
         if constexpr( !Closure<CL>::LINEAR && Closure<CL>::NS < 4 )
             if( which == KERNEL_CHECK_SMALL ) return (void*)&k_check_small<CL, NTM>;
         if( which == KERNEL_UPDATE_SMALL ) return (void*)&k_update_small<CL, true, NTM>;
@@ -53,6 +54,15 @@ template <int CL> void* kernel_of( int group, int which ) {
             return nullptr;
         case KERNEL_UPDATE_PLAIN_WALL:
             if constexpr( Closure<CL>::NS == 4 ) return (void*)&k_update<CL, false, true, false>;
+            return nullptr;
+        case KERNEL_UPDATE_MMA:
+        case KERNEL_UPDATE_MMA_PLAIN:
+            if constexpr( CL == 1 ) {
+                const bool fin = which == KERNEL_UPDATE_MMA;
+                if( group == UPD_TILES[0] ) return fin ? (void*)&k_update_mma<CL, true, UPD_TILES[0]> : (void*)&k_update_mma<CL, false, UPD_TILES[0]>;
+                if( group == UPD_TILES[1] ) return fin ? (void*)&k_update_mma<CL, true, UPD_TILES[1]> : (void*)&k_update_mma<CL, false, UPD_TILES[1]>;
+                if( group == UPD_TILES[2] ) return fin ? (void*)&k_update_mma<CL, true, UPD_TILES[2]> : (void*)&k_update_mma<CL, false, UPD_TILES[2]>;
+            }
             return nullptr;
         case KERNEL_INIT:
             if( group == 32 ) return (void*)&k_init<CL, 32>;

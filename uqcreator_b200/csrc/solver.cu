@@ -31,6 +31,7 @@
 #include "newton_batch.cuh"
 #include "newton_tiny.cuh"
 #include "small_cells.cuh"
+#include "update_mma.cuh"
 #include "uqc.h"
 
 using namespace uqc;
@@ -83,6 +84,8 @@ struct uqc_solver {
     int closureBlock = 256, closureGrid = 0, updateBlock = 256, updateGrid = 0, auxGrid = 0, auxBlock = 256;
     size_t closureSmem = 0, updateSmem = 0, initSmem = 0, mvSmem = 0, checkSmem = 0;
     int checkBlock = 256, checkGrid = 0;
+    int updateNodes = 0, updateLd = 0;    // k_update_mma: nodes per chunk, row stride of its table
+    double* d_phiWfP = nullptr;
     void *checkFn = nullptr, *updateFn = nullptr;    // the check kernel, and the update kernel the steps launch
     int* d_activeList = nullptr;    // cells that need Newton: two lists (running step, next step)
     double* d_cellDt  = nullptr;    // per cell: CFL step of its nodal states
@@ -286,6 +289,9 @@ KParams make_params( const uqc_solver* h ) {
     P.ldT          = ( h->tab.nQ + 3 ) & ~3;
     P.pairSlots    = h->d_pairSlots;
     P.tinyTab      = h->d_tinyTab;
+    P.phiWfP       = h->d_phiWfP;
+    P.ldP          = h->updateLd;
+    P.updNodes     = h->updateNodes;
     P.tabInSmem    = h->newtonTab ? 1 : 0;
     P.tablesInSmem = h->tablesInSmem;
     P.area         = h->d_area;
@@ -670,17 +676,60 @@ void plan_newton( uqc_solver* h, int maxSmem ) {
     }
 }
 
+// k_update_mma for the 2-D Euler states (no walls) of up to 64 moments (k_update
+// / k_update_mma, us: 10 moments, 36 nodes, 100k cells 351 / 223; 21 moments, 100
+// nodes, 200k cells 1150 / 811; 35 moments, 512 nodes, 262k cells 8950 / 5020): the
+// table whole where two CTAs' share of shared memory holds it beside the fluxes,
+// else in chunks of 64 nodes.
+void plan_update_mma( uqc_solver* h, int maxSmem ) {
+    const int nT = h->tab.nT, nQ = h->tab.nQ, nQ4 = ( nQ + 3 ) & ~3;
+    if( h->cfg.closure != 1 || h->d_bndNormal != nullptr || h->mesh.nFaces != 3 ) return;
+    for( int tiles : UPD_TILES ) {
+        if( nT > 8 * tiles ) continue;
+        const int warps = h->updateWarpsOpt > 0 ? std::min( h->updateWarpsOpt, 8 ) : 8;
+        int chunk       = nQ4;
+        size_t smem     = update_mma_doubles( h->nS, nQ, chunk, tiles, warps ) * sizeof( double );
+        if( smem > size_t( maxSmem ) / 2 - 1024 ) {
+            chunk = 64;
+            if( chunk >= nQ ) return;
+            smem = update_mma_doubles( h->nS, nQ, chunk, tiles, warps ) * sizeof( double );
+        }
+        void* fn = pick( h->cfg.closure, tiles, update_test_on( h ) ? KERNEL_UPDATE_MMA : KERNEL_UPDATE_MMA_PLAIN );
+        allow_dynamic_smem( fn );
+        int occ = 0;
+        CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, fn, 32 * warps, smem ) );
+        if( occ < 1 ) return;
+        h->updateFn    = fn;
+        h->updateBlock = 32 * warps;
+        h->updateSmem  = smem;
+        h->updateNodes = chunk;
+        h->updateLd    = upd_ld( tiles );
+        h->updateGrid  = std::min( occ * h->numSMs, std::max( 1, ( h->mesh.nCells + 2 * warps - 1 ) / ( 2 * warps ) ) );
+        if( h->updateGrid > h->blockPartialCap ) {
+            if( h->d_blockPartial ) cudaFree( h->d_blockPartial );
+            h->d_blockPartial  = dalloc<double>( size_t( h->updateGrid ) );
+            h->blockPartialCap = h->updateGrid;
+        }
+        if( !h->d_phiWfP ) {
+            std::vector<double> tab( size_t( nQ4 ) * h->updateLd, 0.0 );
+            for( int k = 0; k < nQ; ++k )
+                for( int i = 0; i < nT; ++i ) tab[size_t( k ) * h->updateLd + i] = h->tab.phiWf[size_t( k ) * nT + i];
+            h->d_phiWfP = dupload( tab );
+        }
+        return;
+    }
+}
+
 // The several-lanes-per-cell check and update kernels instead of the warp-per-
 // cell ones, where an instance holds the moments in a lane's registers. Update,
 // warp per cell / lanes (us): Burgers, 10 moments, 20k cells 43 / 25, 200k 336 / 121;
 // adaptive shallow water, 50k cells 55 / 29, 1M 1063 / 410 (check 1177 / 472);
-// 2-D Euler, 6 moments, 10k cells 36 / 32, 100k 266 / 138, 10 moments, 100k cells
-// 351 / 294 but 10k cells 46 / 52 (with 10 moments of four states a lane needs all
-// its registers and an SM holds eight warps: only where the mesh is large enough).
+// 2-D Euler, 6 moments, 10k cells 36 / 32, 100k 266 / 138 (k_update_mma 29 / 147; 3
+// moments 28 / 24 and 115 / 88, 10 moments, 100k cells 223 / 292: there a lane needs
+// all its registers and an SM holds eight warps).
 void plan_small( uqc_solver* h ) {
     const int cl = h->cfg.closure, nT = h->tab.nT;
     if( h->d_bndNormal != nullptr || h->mesh.nFaces != ( h->nS == 4 ? 3 : 2 ) ) return;
-    if( h->nS == 4 && nT > SMALL_NT[0] && h->mesh.nCells < 20000 ) return;
     for( int ntm : SMALL_NT ) {
         if( nT > ntm ) continue;
         const size_t table = size_t( h->tab.nQ ) * h->ld * sizeof( double );
@@ -795,7 +844,7 @@ void plan_launches( uqc_solver* h ) {
         }
     }
     const int ug = h->auxBlock / h->group;    // groups per CTA of the init / mean-variance kernels
-    h->initSmem   = size_t( ug ) * ( size_t( nS ) * nQ + 8 ) * sizeof( double );
+    h->initSmem   = size_t( ug ) * init_group_doubles( nS, nT, nQ, h->group ) * sizeof( double );
     h->mvSmem     = size_t( ug ) * ( 2 * size_t( nS ) * nQ + 8 ) * sizeof( double );
     for( int which : {2, 3} ) {
         size_t sm = which == 2 ? h->initSmem : h->mvSmem;
@@ -817,6 +866,7 @@ void plan_launches( uqc_solver* h ) {
         CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kk, h->checkBlock, h->checkSmem ) );
         h->checkGrid = std::min( std::max( 1, occ ) * h->numSMs, std::max( 1, ( h->mesh.nCells + warps - 1 ) / warps ) );
     }
+    plan_update_mma( h, maxSmem );
     plan_small( h );
     plan_newton( h, maxSmem );
     plan_mixed( h, maxSmem );
@@ -1038,7 +1088,7 @@ void release( uqc_solver* h ) {
                     (void*)h->d_unitN, (void*)h->d_scaledN, (void*)h->d_nbr, (void*)h->d_boundary, (void*)h->d_u, (void*)h->d_lam,
                     (void*)h->d_bndNormal, (void*)h->d_uQ, (void*)h->d_uOld0, (void*)h->d_blockPartial, (void*)h->d_chunkPartial, (void*)h->d_level, (void*)h->d_status,
                     (void*)h->d_iters, (void*)h->d_ctl, (void*)h->d_xLam, (void*)h->d_xU, (void*)h->d_xNt, (void*)h->d_xStatus,
-                    (void*)h->d_xIters, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_phiT, (void*)h->d_pairSlots, (void*)h->d_tinyTab, (void*)h->d_fallbackList,
+                    (void*)h->d_xIters, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_phiT, (void*)h->d_pairSlots, (void*)h->d_tinyTab, (void*)h->d_phiWfP, (void*)h->d_fallbackList,
                     (void*)h->d_factorStore, (void*)h->d_factorLevel, (void*)h->d_gStore, (void*)h->d_v2Lists,
                     (void*)h->d_chordIters, (void*)h->d_qTiles, (void*)h->d_sendCells, (void*)h->d_filter, (void*)h->d_lassoParam,
                     (void*)h->d_lassoL1} )
