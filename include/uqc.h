@@ -54,7 +54,7 @@ enum uqc_layout { UQC_LAYOUT_REF = 0, UQC_LAYOUT_STATE_MAJOR = 1 };
  *            factor not positive definite, line-search or iteration limit)
  *            continue from their last accepted duals in the FP64 form. Where
  *            the FP64 form's kernel is the faster one it runs by default:
- *            systems of at most 6 duals, the 2-D Euler closure of up to 48 duals
+ *            systems "closure_tiny" takes, the 2-D Euler closure of up to 48 duals
  *            or without the tensor-core rounds, and its closure-only calls. */
 enum uqc_precision { UQC_FP64 = 0, UQC_MIXED = 1 };
 
@@ -174,7 +174,8 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
  *                    kernel (default 16) and the mixed form's chord kernel
  *                    (default 16), each capped by shared memory; 0 = default.
  *   "closure_tiny"   systems of at most 6 duals per cell (states x moments)
- *                    on at most 64 nodes: -1 (default) / 1: a kernel with the
+ *                    on at most 64 nodes, and of at most 10 on meshes of up
+ *                    to 32,768 cells (1: of any size): -1 (default) / 1: a kernel with the
  *                    Newton of each cell on one warp (a lane per entry of the
  *                    system, every lane solving it itself), in both
  *                    precisions (FP64 arithmetic);

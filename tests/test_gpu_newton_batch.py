@@ -61,17 +61,20 @@ def test_closure_of_a_batch(degree, nquad, dim_xi, n):
 
 
 @pytest.mark.parametrize("toml", [
-    W.burgers1d(ncells=90, degree=6, nquad=9, eps=EPS),      # 7 duals: more than the register Newton takes
+    W.burgers1d(ncells=90, degree=6, nquad=9, eps=EPS),      # 7 duals
     W.burgers1d(ncells=90, degree=9, nquad=40, eps=EPS),     # 55 pairs, 7 row tiles
     W.burgers1d(ncells=90, degree=10, nquad=21, eps=EPS),    # 66 pairs: the second shape
     W.burgers1d(ncells=90, degree=14, nquad=30, eps=EPS),    # 120 pairs, its largest
     W.shallow_water1d(ncells=90, max_degree=3, nquad=7, eps=EPS),
     W.shallow_water1d(ncells=90, max_degree=9, nquad=30, eps=EPS),
 ], ids=["burgers_7", "burgers_10", "burgers_11", "burgers_15", "sw_8", "sw_20"])
-def test_closure_of_small_systems(toml):
+@pytest.mark.parametrize("tiny", [-1, 0])
+def test_closure_of_small_systems(toml, tiny):
     """One and two states, odd numbers of blocks: statuses and the convergence
-    test as above, with different moment counts per cell where there are levels."""
+    test as above, with different moment counts per cell where there are levels;
+    up to 10 duals with the kernel of tiny systems and without it."""
     o, s = Oracle(toml), Solver(toml)
+    s.set_option("closure_tiny", tiny)
     o.init_state()
     u, lam0, _ = o.get_state()
     nt = np.array(s.n_total_levels, dtype=np.uint32)[np.arange(len(u)) % s.n_levels]

@@ -37,7 +37,7 @@ template <int CL> void* kernel_of( int group, int which ) {
             if( group == 256 ) return (void*)&k_closure<CL, 256, double>;
             return nullptr;
         case KERNEL_CLOSURE_TINY:
-            if constexpr( !Closure<CL>::LINEAR ) return (void*)&k_newton_tiny<CL>;
+            if constexpr( !Closure<CL>::LINEAR ) return group == SMALL_N ? (void*)&k_newton_tiny<CL, SMALL_N> : (void*)&k_newton_tiny<CL, TINY_N>;
             return nullptr;
         case KERNEL_CLOSURE_MIXED:
             if constexpr( !Closure<CL>::LINEAR ) {

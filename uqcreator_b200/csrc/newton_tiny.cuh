@@ -1,4 +1,4 @@
-// FP64 Newton closure of tiny systems (n = nS nT <= TINY_N duals, at most 64
+// FP64 Newton closure of tiny systems (n = nS nT <= 6 or 10 duals, at most 64
 // nodes), a warp per cell.
 //
 // A step of a small mesh lasts as long as its slowest cell's Newton, so what
@@ -6,10 +6,10 @@
 // node k (and k + 32): nodal duals, U and DU with one exponential and one
 // reciprocal. The sums over the nodes are not butterflies (27 values through
 // five levels of shuffles, some 400 instructions) but columns: lane e owns one
-// entry of the lower triangle of the Hessian or of the gradient and runs over
-// the nodes with its column of a constant table, Q(k, e) = phi_ki phi_kj wt_k or
-// phi_ki wt_k, in four partial sums; the 27 results go through shared memory to
-// every lane, and every lane eliminates the system for itself (L D L^T, one
+// entry of the lower triangle of the Hessian or of the gradient (two with ten
+// duals) and runs over the nodes with its column of a constant table, Q(k, e) =
+// phi_ki phi_kj wt_k or phi_ki wt_k, in four partial sums; the results go through
+// shared memory to every lane, and every lane eliminates the system for itself (L D L^T, one
 // reciprocal per pivot, the gradient as an extra row). Gradient and Hessian come
 // from the same pass, so a trial that is accepted has its next direction's
 // matrix at hand. The iteration, tests and line search are newton_cell's
@@ -19,43 +19,52 @@
 // slots). Burgers, 5 duals, 20 nodes: closure phase of a step on 500 cells 35 ->
 // 20 us (with its launches and events), on 20k cells 65 -> 31; the whole solve of
 // 500 cells 42 -> 23 us a step. Two CTAs of four warps per SM: the system, its
-// matrix and the duals stay in 240 registers (at 168 they spill).
+// matrix and the duals of 6 stay in 240 registers (at 168 they spill); the instance
+// of 10 spills 276 B, mostly the basis values of the lane's nodes, and still shortens
+// the chain: Burgers, 10 duals, 40 nodes, a step on 500 cells 46 -> 33, on 20k 63 -> 56.
 #pragma once
 #include "ipm_kernels.cuh"
 
 namespace uqc {
 
-constexpr int TINY_N = 6, TINY_H = TINY_N * ( TINY_N + 1 ) / 2, TINY_MAX_NODES = 64;
+// Instances: systems of up to TINY_N or SMALL_N duals.
+constexpr int TINY_N = 6, SMALL_N = 10, TINY_MAX_NODES = 64, SMALL_CELLS = 32768;
+__host__ __device__ constexpr int tiny_h( int TN ) { return TN * ( TN + 1 ) / 2; }           // Hessian entries
+__host__ __device__ constexpr int tiny_sums( int TN ) { return tiny_h( TN ) + TN; }
+__host__ __device__ constexpr int tiny_cols( int TN ) { return ( tiny_sums( TN ) + 31 ) & ~31; }    // table columns
 
 // Duals in basis-major order a = i nS + s, so that a level's duals are a prefix
-// whatever its moment count. Table entry (k, e): e < TINY_H the pair a >= b with
+// whatever its moment count. Table entry (k, e): e < tiny_h the pair a >= b with
 // e = a (a + 1) / 2 + b, then the gradient rows; phi and wt as in KParams.
-inline double tiny_entry( int nS, int nT, const double* phiRow, double wt, int e ) {
-    if( e < TINY_H ) {
+inline double tiny_entry( int TN, int nS, int nT, const double* phiRow, double wt, int e ) {
+    if( e < tiny_h( TN ) ) {
         int a = 0;
         while( ( a + 1 ) * ( a + 2 ) / 2 <= e ) ++a;
         const int i = a / nS, j = ( e - a * ( a + 1 ) / 2 ) / nS;
         return i < nT ? phiRow[i] * phiRow[j] * wt : 0.0;
     }
-    const int i = ( e - TINY_H ) / nS;
-    return e < TINY_H + TINY_N && i < nT ? phiRow[i] * wt : 0.0;
+    const int i = ( e - tiny_h( TN ) ) / nS;
+    return e < tiny_sums( TN ) && i < nT ? phiRow[i] * wt : 0.0;
 }
 
-// doubles of a warp's shared memory: DU blocks and U at the nodes, the 32 sums,
+// doubles of a warp's shared memory: DU blocks and U at the nodes, the sums,
 // moments, moment sums, reduction scratch
-__host__ __device__ inline int tiny_warp_doubles( int nS, int NP, int nQ ) { return ( NP + nS ) * nQ + 32 + 2 * 8 + 32; }
+__host__ __device__ inline int tiny_warp_doubles( int TN, int nS, int NP, int nQ ) { return ( ( NP + nS ) * nQ + tiny_cols( TN ) + 2 * 12 + 32 + 1 ) & ~1; }
 
-template <int CL> __global__ void __launch_bounds__( 128, 2 ) k_newton_tiny( KParams P, int mode ) {
-    constexpr int NS = Closure<CL>::NS, NP = Closure<CL>::NP, TN = TINY_N, TT = ( TN + NS - 1 ) / NS;
+template <int CL, int TN> __global__ void __launch_bounds__( 128, 2 ) k_newton_tiny( KParams P, int mode ) {
+    constexpr int NS = Closure<CL>::NS, NP = Closure<CL>::NP, TT = ( TN + NS - 1 ) / NS;
+    constexpr int TH = tiny_h( TN ), SUMS = tiny_sums( TN ), COLS = tiny_cols( TN );
+    // whole rounds of 32 sums, a lane each; up to two left over are spread over the lanes
+    constexpr int REST = SUMS % 32 <= 2 ? SUMS % 32 : 0, ROUNDS = ( SUMS - REST + 31 ) / 32;
     extern __shared__ __align__( 16 ) double smem[];
     if( mode == 1 && !P.ctl->active ) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nWarps = blockDim.x >> 5;
-    for( int i = threadIdx.x; i < 32 * P.nQ; i += blockDim.x ) smem[i] = P.tinyTab[i];
-    const double* Q = smem + lane;    // the lane's column, row stride 32
-    double* nod     = smem + 32 * P.nQ + warp * tiny_warp_doubles( NS, NP, P.nQ );    // DU (b nQ + k), then U (s nQ + k)
+    for( int i = threadIdx.x; i < COLS * P.nQ; i += blockDim.x ) smem[i] = P.tinyTab[i];
+    const double* Q = smem + lane;    // the lane's columns, row stride COLS
+    double* nod     = smem + COLS * P.nQ + warp * tiny_warp_doubles( TN, NS, NP, P.nQ );    // DU (b nQ + k), then U (s nQ + k)
     double* uk      = nod + NP * P.nQ;
     double* sums    = uk + NS * P.nQ;
-    double *uhS = sums + 32, *msS = uhS + 8, *red = msS + 8;
+    double *uhS = sums + COLS, *msS = uhS + 12, *red = msS + 12;
     // the lane's nodes
     double ph[2][TT];
 #pragma unroll
@@ -65,21 +74,23 @@ template <int CL> __global__ void __launch_bounds__( 128, 2 ) k_newton_tiny( KPa
             const int k = lane + 32 * q;
             ph[q][i]    = k < P.nQ && i < P.nT ? P.phi[size_t( k ) * P.ld + i] : 0.0;
         }
-    // the lane's sum: Hessian entry (a, b) of the blocks (s, t), or gradient row a
-    const double* src = uk;
-    int msAt          = -1;    // place of its moment sum in msS (state-major)
-    {
-        if( lane < TINY_H ) {
+    // a sum's source: Hessian entry (a, b) of the blocks (s, t), or gradient row a;
+    // and the place of a gradient row's moment sum in msS (state-major)
+    auto source = [&]( int e, int& msAt ) {
+        msAt = -1;
+        if( e < TH ) {
             int a = 0;
-            while( ( a + 1 ) * ( a + 2 ) / 2 <= lane ) ++a;
-            src = nod + pair_index<NS>( a % NS, ( lane - a * ( a + 1 ) / 2 ) % NS ) * P.nQ;
+            while( ( a + 1 ) * ( a + 2 ) / 2 <= e ) ++a;
+            return (const double*)( nod + pair_index<NS>( a % NS, ( e - a * ( a + 1 ) / 2 ) % NS ) * P.nQ );
         }
-        else if( lane < TINY_H + TN ) {
-            const int a = lane - TINY_H;
-            src         = uk + ( a % NS ) * P.nQ;
-            if( a / NS < P.nT ) msAt = ( a % NS ) * P.nT + a / NS;
-        }
-    }
+        const int a = min( e - TH, TN - 1 );
+        if( e < SUMS && a / NS < P.nT ) msAt = ( a % NS ) * P.nT + a / NS;
+        return (const double*)( uk + ( a % NS ) * P.nQ );
+    };
+    const double* src[ROUNDS];
+    int msAt[ROUNDS];
+#pragma unroll
+    for( int q = 0; q < ROUNDS; ++q ) src[q] = source( lane + 32 * q, msAt[q] );
     __syncthreads();
     const Grp<32> grp{lane, 0};
     const int ldc    = NS * P.nT;
@@ -97,7 +108,7 @@ template <int CL> __global__ void __launch_bounds__( 128, 2 ) k_newton_tiny( KPa
         const int cell = alist ? alist[item] : item;
         const int lev = P.level ? int( P.level[cell] ) : P.nLevels - 1;
         const int nTj = P.nTotalCell ? int( P.nTotalCell[cell] ) : P.nTLevel[lev], n = NS * nTj;
-        double lam[TN], lamN[TN], uh[TN], d[TN], h[TINY_H], g[TN];
+        double lam[TN], lamN[TN], d[TN], h[TH], g[TN];
         bool bad = false;
         if( lane < ldc ) {
             const double a = P.lam[size_t( cell ) * ldc + lane], b = P.u[size_t( cell ) * ldc + lane];
@@ -109,7 +120,6 @@ template <int CL> __global__ void __launch_bounds__( 128, 2 ) k_newton_tiny( KPa
         for( int a = 0; a < TN; ++a ) {
             const int s = a % NS, i = a / NS;
             lam[a] = a < n ? P.lam[size_t( cell ) * ldc + s * P.nT + i] : 0.0;
-            uh[a]  = a < n ? P.u[size_t( cell ) * ldc + s * P.nT + i] : 0.0;
         }
         // U and DU at the duals x, Hessian h and gradient g there; ||g||
         auto evaluate = [&]( const double( &x )[TN] ) {
@@ -131,25 +141,41 @@ template <int CL> __global__ void __launch_bounds__( 128, 2 ) k_newton_tiny( KPa
                 }
             }
             __syncwarp();
-            double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-            int k = 0;
-            for( ; k + 3 < P.nQ; k += 4 ) {
-                a0 = fma( src[k], Q[32 * k], a0 );
-                a1 = fma( src[k + 1], Q[32 * k + 32], a1 );
-                a2 = fma( src[k + 2], Q[32 * k + 64], a2 );
-                a3 = fma( src[k + 3], Q[32 * k + 96], a3 );
+#pragma unroll
+            for( int q = 0; q < ROUNDS; ++q ) {
+                double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+                const double *x = src[q], *w = Q + 32 * q;
+                int k = 0;
+                for( ; k + 3 < P.nQ; k += 4, x += 4, w += 4 * COLS ) {
+                    a0 = fma( x[0], w[0], a0 );
+                    a1 = fma( x[1], w[COLS], a1 );
+                    a2 = fma( x[2], w[2 * COLS], a2 );
+                    a3 = fma( x[3], w[3 * COLS], a3 );
+                }
+                for( ; k < P.nQ; ++k, ++x, w += COLS ) a0 = fma( x[0], w[0], a0 );
+                const double sum    = ( a0 + a1 ) + ( a2 + a3 );
+                sums[lane + 32 * q] = sum;
+                if( msAt[q] >= 0 ) msS[msAt[q]] = sum;
             }
-            for( ; k < P.nQ; ++k ) a0 = fma( src[k], Q[32 * k], a0 );
-            const double sum = ( a0 + a1 ) + ( a2 + a3 );
-            sums[lane]       = sum;
-            if( msAt >= 0 ) msS[msAt] = sum;
+#pragma unroll
+            for( int e = SUMS - REST; e < SUMS; ++e ) {
+                int at;
+                const double* x = source( e, at );
+                double v        = 0.0;
+                for( int k = lane; k < P.nQ; k += 32 ) v = fma( x[k], smem[k * COLS + e], v );
+                for( int o = 16; o > 0; o >>= 1 ) v += __shfl_xor_sync( 0xffffffffu, v, o );
+                if( lane == 0 ) {
+                    sums[e] = v;
+                    if( at >= 0 ) msS[at] = v;
+                }
+            }
             __syncwarp();
 #pragma unroll
-            for( int e = 0; e < TINY_H; ++e ) h[e] = sums[e];
+            for( int e = 0; e < TH; ++e ) h[e] = sums[e];
             double s0 = 0.0, s1 = 0.0;
 #pragma unroll
             for( int a = 0; a < TN; ++a ) {
-                g[a] = a < n ? sums[TINY_H + a] - uh[a] : 0.0;
+                g[a] = a < n ? sums[TH + a] - uhS[( a % NS ) * P.nT + a / NS] : 0.0;
                 ( a & 1 ? s1 : s0 ) = fma( g[a], g[a], a & 1 ? s1 : s0 );
             }
             return sqrt( s0 + s1 );
@@ -176,10 +202,12 @@ template <int CL> __global__ void __launch_bounds__( 128, 2 ) k_newton_tiny( KPa
             for( int j = TN - 1; j >= 0; --j ) {
                 d[j] = 0.0;
                 if( j < n ) {
-                    double v = g[j];
+                    // (L D L^T x = b after the forward pass: x_j = y_j / D_j - sum_i l_ij x_i,
+                    // with h holding l_ij D_j)
+                    double v = g[j], z = 0.0;
 #pragma unroll
-                    for( int i = j + 1; i < TN; ++i ) v = fma( -h[i * ( i + 1 ) / 2 + j], d[i], v );
-                    d[j] = v * r[j];
+                    for( int i = j + 1; i < TN; ++i ) ( i & 1 ? z : v ) = fma( -h[i * ( i + 1 ) / 2 + j], d[i], i & 1 ? z : v );
+                    d[j] = ( v + z ) * r[j];
                 }
             }
             return pd;

@@ -52,7 +52,7 @@ struct uqc_solver {
     double* d_chunkPartial = nullptr;  // uqc_step_host's chunked update: a partial per CTA and launch
     int chunkPartialCap    = 0;
     bool closureTiny = false;          // planned: the Newton of tiny systems (k_newton_tiny)
-    int tinyGrid     = 0;
+    int tinyGrid = 0, tinyN = 0;
     size_t tinySmem  = 0;
     double* d_tinyTab = nullptr;
     // FP64 closure of large systems: k_newton's instance (a KernelId, 0: k_closure) and launch shape
@@ -785,20 +785,26 @@ void plan_launches( uqc_solver* h ) {
     int occ = 0;
     CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kc, h->closureBlock, h->closureSmem ) );
     h->closureGrid = std::max( 1, occ ) * h->numSMs;
-    // tiny systems (n <= TINY_N duals, at most 64 nodes): k_newton_tiny, a warp per cell
-    h->closureTiny =
-        h->tinyOpt != 0 && h->closureGroup == 32 && n <= size_t( TINY_N ) && nQ <= TINY_MAX_NODES && !closure_linear( cl );
+    // tiny systems (at most 64 nodes): k_newton_tiny, a warp per cell. Up to TINY_N duals
+    // always; up to SMALL_N on meshes of at most SMALL_CELLS cells, where the chain of one
+    // cell counts and not the packing: closure phase of a step in us, k_newton / tiny, 10
+    // duals: Burgers, 500 cells 46 / 33, 20k cells 63 / 56 (first step 529 / 488), 200k cells
+    // 361 / 377; shallow water, 50k cells, 48 / 43 but its first step 173 / 213
+    h->closureTiny = h->tinyOpt != 0 && h->closureGroup == 32 && nQ <= TINY_MAX_NODES && !closure_linear( cl ) &&
+                     ( n <= size_t( TINY_N ) || ( n <= size_t( SMALL_N ) && ( h->tinyOpt == 1 || h->mesh.nCells <= SMALL_CELLS ) ) );
     if( h->closureTiny ) {
-        void* kt    = pick( cl, 32, KERNEL_CLOSURE_TINY );
-        h->tinySmem = ( size_t( 32 ) * nQ + 4 * size_t( tiny_warp_doubles( nS, closure_np( cl ), nQ ) ) ) * sizeof( double );
+        h->tinyN    = n <= size_t( TINY_N ) ? TINY_N : SMALL_N;
+        void* kt    = pick( cl, h->tinyN, KERNEL_CLOSURE_TINY );
+        h->tinySmem = ( size_t( tiny_cols( h->tinyN ) ) * nQ + 4 * size_t( tiny_warp_doubles( h->tinyN, nS, closure_np( cl ), nQ ) ) ) * sizeof( double );
         allow_dynamic_smem( kt );
         CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kt, 128, h->tinySmem ) );
         h->tinyGrid = std::max( 1, occ ) * h->numSMs;
         if( !h->d_tinyTab ) {
-            std::vector<double> tab( size_t( 32 ) * nQ );
+            const int cols = tiny_cols( h->tinyN );
+            std::vector<double> tab( size_t( cols ) * nQ );
             for( int k = 0; k < nQ; ++k )
-                for( int e = 0; e < 32; ++e )
-                    tab[size_t( 32 ) * k + e] = tiny_entry( nS, nT, &h->tab.phi[size_t( k ) * nT], h->padWt[k], e );
+                for( int e = 0; e < cols; ++e )
+                    tab[size_t( cols ) * k + e] = tiny_entry( h->tinyN, nS, nT, &h->tab.phi[size_t( k ) * nT], h->padWt[k], e );
             h->d_tinyTab = dupload( tab );
         }
     }
@@ -1130,7 +1136,7 @@ void launch_closure( uqc_solver* h, KParams& P, int mode ) {
         // tiny systems: the FP64 register Newton in both precisions (the mixed
         // form's FP32 Hessian saves nothing at this size)
         void* args[] = {&P, &mode};
-        launch( h, pick( h->cfg.closure, 32, KERNEL_CLOSURE_TINY ), h->tinyGrid, 128, h->tinySmem, args );
+        launch( h, pick( h->cfg.closure, h->tinyN, KERNEL_CLOSURE_TINY ), h->tinyGrid, 128, h->tinySmem, args );
         return;
     }
     if( mode == 1 && P.gStore ) {
