@@ -86,6 +86,21 @@ def test_reformed_inverse_matches_fp64(form):
     assert worst <= 2e-3, worst
 
 
+@pytest.mark.parametrize("degree,nquad,dim_xi", [(1, 3, 2), (12, 16, 1), (5, 10, 2), (21, 24, 1)],
+                         ids=["n12", "n52", "n84", "n88"])
+def test_inverse_by_pivot_pairs(degree, nquad, dim_xi):
+    """The sweep kernel where the matrix ends inside a warp's rows, in a later
+    warp's, and fills them all (22 rows a warp; condition numbers up to 430 at
+    these states, so the bound is the one above)."""
+    s = _state_after_steps(W.euler2d(nx=8, ny=3, degree=degree, nquad=nquad, dim_xi=dim_xi))
+    _, lam, _ = s.download_state()
+    phi, _, _, w = s.tables()
+    cells = np.arange(s.n_cells)
+    for c, hinv in zip(cells, s.debug_mixed_inverse(cells, 2)):
+        ref = np.linalg.inv(_fp64_hessian(phi, w, dim_xi, lam[c]))
+        assert np.linalg.norm(hinv - ref) <= 2e-3 * np.linalg.norm(ref)
+
+
 def test_tensor_and_cuda_core_inverses_agree():
     s = _state_after_steps(W.euler2d(nx=12, ny=4, degree=3, nquad=6))
     cells = np.arange(s.n_cells)

@@ -849,31 +849,34 @@ template <int CL, bool RAW> __global__ void __launch_bounds__( 256, 1 ) k_invert
 // Rows of a cell's matrix per warp and columns per lane of k_invert_sweep:
 // four warps per cell hold the n x n matrix (n <= 4 SWEEP_RG) in registers,
 // warp g rows [SWEEP_RG g, SWEEP_RG (g + 1)), lane l columns l, l + 32, l + 64.
-constexpr int SWEEP_RG = 21, SWEEP_CW = 3;
+constexpr int SWEEP_RG = 22, SWEEP_CW = 3;    // rows even: a pair of pivots lies in one warp's rows
 
 // floats per cell of k_invert_sweep's shared memory: the raw values (rounded
 // up to 16 bytes), two pivot-row buffers, two ints; a multiple of 4 floats
 __host__ __device__ inline size_t sweep_raw_floats( int pairs, int NP ) { return ( size_t( pairs ) * NP + 3 ) & ~size_t( 3 ); }
 // a pivot-row buffer: 32 SWEEP_CW columns (those beyond the matrix hold
-// zeros) and the pivot itself at index 32 SWEEP_CW
+// zeros) and the row's entries of the pivot block at index 32 SWEEP_CW
 constexpr int SWEEP_PR = 32 * SWEEP_CW + 4;
 // a pivot-column buffer: the same values by row group, SWEEP_PG floats per
 // group (SWEEP_RG rounded up to 4), so that a warp reads its rows' column
 // values in 16-byte loads
 constexpr int SWEEP_PG = ( SWEEP_RG + 3 ) & ~3, SWEEP_PC = 4 * SWEEP_PG;
 __host__ __device__ inline size_t sweep_ws_floats( int pairs, int NP ) {
-    return sweep_raw_floats( pairs, NP ) + 2 * SWEEP_PR + 2 * SWEEP_PC + 8;
+    return sweep_raw_floats( pairs, NP ) + 4 * SWEEP_PR + 4 * SWEEP_PC + 8;    // two buffers of two pivot rows
 }
 
 // H^-1 of the cells of re-factor list `round` from the raw values k_hess_tc
 // left in their store slots, by the sweep operator (Gauss-Jordan on a
-// symmetric matrix: sweeping pivot k maps a_kk -> -1/a_kk, a_ik -> a_ik / a_kk,
-// a_ij -> a_ij - a_ik a_kj / a_kk; after all n pivots the matrix is -H^-1).
-// The matrix stays symmetric, so column k is row k: one warp publishes the
-// pivot row in shared memory, one named barrier per pivot, and every thread
-// updates its 21 x 3 register block with one FMA per element. No pivoting:
-// H is symmetric positive definite, and a pivot that is not positive (FP32
-// factor not positive definite) sends the cell to the FP64 fallback list.
+// symmetric matrix) on pairs of pivots p = (k, k + 1) with the block P: A_pp ->
+// -P^-1, A_ip -> A_ip P^-1, A_ij -> A_ij - A_ip P^-1 A_pj; after all pairs the matrix is
+// -H^-1. The matrix stays symmetric, so the pivot columns are the pivot rows: one
+// warp publishes the two rows in shared memory, one named barrier per pair, and
+// every thread updates its 22 x 3 register block with two FMAs per element. (One
+// pivot at a time, with a barrier, a reciprocal and a publication each: 7190 us for
+// 90,000 cells of 84 duals, pairs 6630; bound by the FMAs of the register block and
+// the shared-memory loads that feed them.) No pivoting: H is symmetric positive definite, and a
+// block that is not (FP32 factor not positive definite) sends the cell to the FP64
+// fallback list.
 template <int CL> __global__ void __launch_bounds__( 512, 1 ) k_invert_sweep( KParams P, int round ) {
     constexpr int NS = Closure<CL>::NS, NP = Closure<CL>::NP;
     constexpr int RG = SWEEP_RG, CW = SWEEP_CW;
@@ -885,9 +888,9 @@ template <int CL> __global__ void __launch_bounds__( 512, 1 ) k_invert_sweep( KP
     const int cg = warp >> 2, g = warp & 3;    // cell group of the CTA, row group of the warp
     const int nT = P.nT, n = NS * nT, pairs = nT * ( nT + 1 ) / 2;
     float* raw  = fsm + size_t( cg ) * sweep_ws_floats( pairs, NP );
-    float* prow = raw + sweep_raw_floats( pairs, NP );    // two pivot-row buffers of SWEEP_PR floats
-    float* pcol = prow + 2 * SWEEP_PR;                     // two pivot-column buffers of SWEEP_PC floats
-    int* misc   = reinterpret_cast<int*>( pcol + 2 * SWEEP_PC );    // [0] item, [1] not positive definite
+    float* prow = raw + sweep_raw_floats( pairs, NP );    // two buffers of two pivot rows (SWEEP_PR floats each)
+    float* pcol = prow + 4 * SWEEP_PR;                     // two buffers of two pivot columns (SWEEP_PC floats each)
+    int* misc   = reinterpret_cast<int*>( pcol + 4 * SWEEP_PC );    // [0] item, [1] not positive definite
     const int bar = 1 + cg, tid = threadIdx.x & 127;
     auto sync = [&]() { asm volatile( "bar.sync %0, 128;" ::"r"( bar ) : "memory" ); };
     const int* list = refactor_list( P, round );
@@ -931,56 +934,77 @@ template <int CL> __global__ void __launch_bounds__( 512, 1 ) k_invert_sweep( KP
         bool bad = false;
         for( int gg = 0; gg < 4; ++gg ) {
 #pragma unroll
-            for( int rr = 0; rr < RG; ++rr ) {
-                const int k = RG * gg + rr;
+            for( int rr = 0; rr < RG; rr += 2 ) {
+                const int k = RG * gg + rr;    // pivots k, k + 1 (beyond n the identity; n may be odd)
                 if( k >= n ) break;
-                float* pr = prow + ( k & 1 ) * SWEEP_PR;
-                float* pc = pcol + ( k & 1 ) * SWEEP_PC;
-                const int kl = k & 31, kq = k >> 5;
+                const int buf = ( k >> 1 ) & 1;
+                float *pr0 = prow + 2 * buf * SWEEP_PR, *pr1 = pr0 + SWEEP_PR;
+                float *pc0 = pcol + 2 * buf * SWEEP_PC, *pc1 = pc0 + SWEEP_PC;
+                const int k1 = k + 1;    // k is even: k and k + 1 are in the same column block
+                const int kq = k >> 5;
                 if( g == gg ) {
-                    // the pivot row; at the pivot p - 1 (so that pr[k] / p = 1 - 1/p,
-                    // the factor that turns column k into a_ik / p), p itself at the end;
-                    // the same values by row group in the column buffer
+                    // the pivot rows; in the pivot columns v - e, so that w = P^-1 v turns
+                    // into e - P^-1 e there and a_ip - f w into the swept f P^-1; P itself
+                    // at the end; the same values by row group in the column buffers
 #pragma unroll
                     for( int q = 0; q < CW; ++q ) {
-                        float v = a[rr][q];
-                        if( lane == kl && q == kq ) {
-                            pr[32 * CW] = v;
-                            v -= 1.f;
+                        const int c = lane + 32 * q;
+                        float x = a[rr][q], y = a[rr + 1][q];
+                        if( q == kq && lane == ( k & 31 ) ) {
+                            pr0[32 * CW] = x;
+                            pr1[32 * CW] = y;
+                            x -= 1.f;
                         }
-                        const int c       = lane + 32 * q;
-                        pr[c]             = v;
-                        const int cg2     = c / RG;
-                        if( cg2 < 4 ) pc[cg2 * SWEEP_PG + ( c - cg2 * RG )] = v;
+                        if( q == kq && lane == ( k1 & 31 ) ) {
+                            pr1[32 * CW + 1] = y;
+                            y -= 1.f;
+                        }
+                        pr0[c]        = x;
+                        pr1[c]        = y;
+                        const int cg2 = c / RG;
+                        if( cg2 < 4 ) {
+                            pc0[cg2 * SWEEP_PG + ( c - cg2 * RG )] = x;
+                            pc1[cg2 * SWEEP_PG + ( c - cg2 * RG )] = y;
+                        }
                     }
                 }
                 sync();
-                const float p    = pr[32 * CW];
-                bad              = bad || !( p > 0.f );
-                const float pinv = __frcp_rn( p );
-                // a_ij -= a_ik a_kj / p (column k: a_ik / p)
-                float sv[CW];
+                const float p00 = pr0[32 * CW], p01 = pr1[32 * CW], p11 = pr1[32 * CW + 1];
+                const float det = fmaf( p00, p11, -p01 * p01 );
+                bad             = bad || !( p00 > 0.f && det > 0.f );
+                const float r   = __frcp_rn( det );
+                const float i00 = p11 * r, i01 = -p01 * r, i11 = p00 * r;
+                // w = P^-1 v of this thread's columns
+                float w0[CW], w1[CW];
 #pragma unroll
-                for( int q = 0; q < CW; ++q ) sv[q] = pr[lane + 32 * q] * pinv;
-                // a_ik of this warp's rows (column k = row k), 16 bytes at a time
-                float f[SWEEP_PG];
-                const float4* pc4 = reinterpret_cast<const float4*>( pc + g * SWEEP_PG );
+                for( int q = 0; q < CW; ++q ) {
+                    const float x = pr0[lane + 32 * q], y = pr1[lane + 32 * q];
+                    w0[q]         = fmaf( i00, x, i01 * y );
+                    w1[q]         = fmaf( i01, x, i11 * y );
+                }
+                // a_ij -= a_ik w0_j + a_i,k+1 w1_j; a_ip of this warp's rows (columns p = rows
+                // p), 16 bytes at a time; in the pivot rows themselves (x - 1, y - 1) not used
+                const float4* f0 = reinterpret_cast<const float4*>( pc0 + g * SWEEP_PG );
+                const float4* f1 = reinterpret_cast<const float4*>( pc1 + g * SWEEP_PG );
 #pragma unroll
                 for( int v4 = 0; v4 < SWEEP_PG / 4; ++v4 ) {
-                    const float4 x = pc4[v4];
-                    f[4 * v4]      = x.x;
-                    f[4 * v4 + 1]  = x.y;
-                    f[4 * v4 + 2]  = x.z;
-                    f[4 * v4 + 3]  = x.w;
+                    const float4 x = f0[v4], y = f1[v4];
+                    const float fx[4] = {x.x, x.y, x.z, x.w}, fy[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                    for( int e = 0; e < 4; ++e ) {
+                        const int i = 4 * v4 + e;
+                        if( i < RG ) {
+#pragma unroll
+                            for( int q = 0; q < CW; ++q ) a[i][q] = fmaf( -fy[e], w1[q], fmaf( -fx[e], w0[q], a[i][q] ) );
+                        }
+                    }
                 }
+                if( g == gg ) {    // the pivot rows: P^-1 v, and -P^-1 in the pivot columns
 #pragma unroll
-                for( int rr2 = 0; rr2 < RG; ++rr2 ) {
-#pragma unroll
-                    for( int q = 0; q < CW; ++q ) a[rr2][q] = fmaf( -f[rr2], sv[q], a[rr2][q] );
-                }
-                if( g == gg ) {    // the pivot row: a_kj / p, and -1/p at the pivot
-#pragma unroll
-                    for( int q = 0; q < CW; ++q ) a[rr][q] = ( lane == kl && q == kq ) ? sv[q] - 1.f : sv[q];
+                    for( int q = 0; q < CW; ++q ) {
+                        a[rr][q]     = q == kq && lane == ( k & 31 ) ? w0[q] - 1.f : w0[q];
+                        a[rr + 1][q] = q == kq && lane == ( k1 & 31 ) ? w1[q] - 1.f : w1[q];
+                    }
                 }
             }
         }

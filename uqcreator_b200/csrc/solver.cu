@@ -483,7 +483,7 @@ void plan_rounds( uqc_solver* h, int maxSmem ) {
         return;
     }
     // inverse kernel: by sweeps in registers (four warps per cell, four cells
-    // per CTA) for n <= 84 after the tensor-core Hessian; else Cholesky and
+    // per CTA) for n <= 88 after the tensor-core Hessian; else Cholesky and
     // triangular inverse, two warps per cell, as many cells (up to 4) as fit
     h->invSweep = mode == 2 && nS * nT <= 4 * SWEEP_RG && nS * nT <= 32 * SWEEP_CW;
     void* ki    = nullptr;
