@@ -20,6 +20,7 @@ CASES = {
     "burgers_17_moments": W.burgers1d(ncells=43, degree=16, nquad=35, tend=10.0),    # the warp-per-cell kernels
     "sw_levels": W.shallow_water1d(ncells=131, max_degree=9, nquad=30, tend=10.0),
     "sw_16_moments": W.shallow_water1d(ncells=70, max_degree=15, nquad=32, tend=10.0),
+    "sw_many_cells": W.shallow_water1d(ncells=250001, max_degree=2, nquad=5, tend=10.0),    # the next cell prefetched
     "euler_3_moments": W.euler2d(nx=7, ny=3, degree=1, nquad=3, tend=10.0),
     "euler_6_moments": W.euler2d(nx=16, ny=5, degree=2, nquad=5, tend=10.0),
     # k_update_mma: two cells a warp (odd counts of cells per warp and mesh), its three

@@ -9,12 +9,14 @@
 // the sums are then exchanged so that lane `sub` keeps the moments i = sub (mod
 // LPC) (LPC - 1 exchanges per LPC moments, a fixed order).
 //
-// Bound by instruction issue and latency (0.45 instructions per cycle and
-// scheduler at 16 warps an SM, registers for the sums allow no more; FP64 pipe
-// 20 %, DRAM 1.1 TB/s). Four lanes per cell: two make the large meshes another
-// 5-15 % faster and the small ones slower, eight the other way round (adaptive
-// shallow water, 1M cells, check 507 / 610 / 722 us at 2 / 4 / 8 lanes, 50k cells 70
-// / 68 / 73). 1M cells: check 1240 -> 472 us, update 1390 -> 410 us.
+// Bound by the latency of a cell's loads and then by issue (0.39 instructions per
+// cycle and scheduler at 16 warps an SM, registers for the sums allow no more; 44 %
+// of the stalls on global loads, FP64 pipe 20-30 %, DRAM 2.2 TB/s): so two nodes at a
+// time, and on large meshes the next cell's state on its way. Four lanes per cell: two
+// made the large meshes another 5-15 % faster and the small ones slower, eight the
+// other way round. Adaptive shallow water, 1M cells: check 1240 us with a warp per
+// cell, 472 with four lanes, 431 with nodes in pairs, 388 with the prefetch; update
+// 1390, 410, 351, 308.
 #pragma once
 #include "ipm_kernels.cuh"
 
@@ -58,7 +60,7 @@ __device__ __forceinline__ void exchange_moments( const double ( &acc )[NS][NTM]
         }
 }
 
-// Sum over the cell's eight lanes, in every one of them.
+// Sum over the cell's lanes, in every one of them.
 __device__ __forceinline__ double cell_sum( double v ) {
     for( int o = LPC / 2; o > 0; o >>= 1 ) v += __shfl_xor_sync( 0xffffffffu, v, o );
     return v;
@@ -66,6 +68,16 @@ __device__ __forceinline__ double cell_sum( double v ) {
 __device__ __forceinline__ double cell_min( double v ) {
     for( int o = LPC / 2; o > 0; o >>= 1 ) v = fmin( v, __shfl_xor_sync( 0xffffffffu, v, o ) );
     return v;
+}
+
+// The next cell's state on its way into L2 while this one's is worked on: a line, or
+// the n doubles at x by the cell's lanes in turn. On meshes of FAR rounds or more, whose
+// state does not stay in L2 (adaptive shallow water, check / update us: 1M cells 431 / 351
+// -> 388 / 308, 200k cells 199 / 120 -> 182 / 108; 50k cells 57 / 27 and without the rule 57 / 29).
+constexpr int FAR = 8;
+__device__ __forceinline__ void prefetch_line( const void* x ) { asm volatile( "prefetch.global.L2 [%0];" ::"l"( x ) ); }
+__device__ __forceinline__ void prefetch_cell( const double* x, int n, int sub ) {
+    for( int i = 16 * sub; i < n; i += 16 * LPC ) prefetch_line( x + i );
 }
 
 // Appends `cell` of the lanes where `on` holds to a device list: one atomic per warp.
@@ -110,6 +122,7 @@ template <int CL, int NTM> __global__ void __launch_bounds__( 256, 2 ) k_check_s
     const int ldc      = NS * P.nT;
     double dtMin       = 1e300;
     const int stride   = gridDim.x * ( blockDim.x / LPC );
+    const bool far     = !listMode && nItems > FAR * stride;
     // whole warps go round together (the exchanges are warp-wide)
     for( int item0 = ( blockIdx.x * blockDim.x + ( threadIdx.x & ~31 ) ) / LPC; item0 < nItems; item0 += stride ) {
         const int item   = item0 + lane / LPC;
@@ -118,6 +131,12 @@ template <int CL, int NTM> __global__ void __launch_bounds__( 256, 2 ) k_check_s
         const double* lam = P.lam + size_t( cell ) * ldc;
         const double* uh  = P.u + size_t( cell ) * ldc;
         if( !listMode && P.finFlag && valid && sub == 0 ) P.finFlag[cell] = 0;
+        if( far && item + stride < nItems ) {
+            const size_t next = size_t( cell ) + stride;
+            prefetch_cell( P.lam + next * ldc, ldc, sub );
+            prefetch_cell( P.u + next * ldc, ldc, sub );
+            prefetch_line( sub & 1 ? (const void*)( P.level + next ) : P.dx + next );
+        }
         const int lev = int( P.level[cell] ), nTj = P.nTLevel[lev];
         bool bad = false;
         for( int idx = sub; idx < ldc; idx += LPC ) bad = bad || !isfinite( lam[idx] ) || !isfinite( uh[idx] );
@@ -138,33 +157,48 @@ template <int CL, int NTM> __global__ void __launch_bounds__( 256, 2 ) k_check_s
         double* uq  = P.uQ + size_t( cell ) * NS * P.nQ;
         double dloc = 1e300;
         const double dx = P.dx[cell];
-        for( int k = sub; k < P.nQ; k += LPC ) {
-            double L[NS], y[NS];
+        // two nodes at a time: the chains of U and dt overlap, the loops' bounds are tested once for both
+        for( int k = sub; k < P.nQ; k += 2 * LPC ) {
+            const bool two = k + LPC < P.nQ;
+            const int k1   = two ? k + LPC : k;    // no second node: the first again, left out of the sums
+            double L[2][NS], y[2][NS];
 #pragma unroll
-            for( int s = 0; s < NS; ++s ) L[s] = 0.0;
-            const double* row = phi + k * P.ld;
+            for( int s = 0; s < NS; ++s ) L[0][s] = L[1][s] = 0.0;
+            const double *row0 = phi + k * P.ld, *row1 = phi + k1 * P.ld;
 #pragma unroll
             for( int i = 0; i < NTM; ++i ) {
                 if( i >= nMax ) break;
-                const double r = row[i];
+                const double r0 = row0[i], r1 = row1[i];
 #pragma unroll
-                for( int s = 0; s < NS; ++s ) L[s] = fma( l[s][i], r, L[s] );
+                for( int s = 0; s < NS; ++s ) {
+                    L[0][s] = fma( l[s][i], r0, L[0][s] );
+                    L[1][s] = fma( l[s][i], r1, L[1][s] );
+                }
             }
-            Closure<CL>::U( L, y, true, P.phys );
+            Closure<CL>::U( L[0], y[0], true, P.phys );
+            Closure<CL>::U( L[1], y[1], true, P.phys );
             if( valid && !bad ) {
                 // a cell that fails the test gets its nodal states from its Newton
 #pragma unroll
-                for( int s = 0; s < NS; ++s ) uq[s * P.nQ + k] = y[s];
+                for( int s = 0; s < NS; ++s ) {
+                    uq[s * P.nQ + k]  = y[0][s];
+                    uq[s * P.nQ + k1] = y[1][s];
+                }
             }
-            const double d = Problem<CL>::dt( y, dx, P.phys );
-            dloc           = d < dloc ? d : dloc;
-            const double* rowW = phiWf + k * P.ld;
+            const double d0 = Problem<CL>::dt( y[0], dx, P.phys ), d1 = Problem<CL>::dt( y[1], dx, P.phys );
+            dloc             = d0 < dloc ? d0 : dloc;
+            dloc             = d1 < dloc ? d1 : dloc;
+            if( !two ) {
+#pragma unroll
+                for( int s = 0; s < NS; ++s ) y[1][s] = 0.0;
+            }
+            const double *w0 = phiWf + k * P.ld, *w1 = phiWf + k1 * P.ld;
 #pragma unroll
             for( int i = 0; i < NTM; ++i ) {
                 if( i >= nMax ) break;
-                const double w = rowW[i];
+                const double x0 = w0[i], x1 = w1[i];
 #pragma unroll
-                for( int s = 0; s < NS; ++s ) acc[s][i] = fma( y[s], w, acc[s][i] );
+                for( int s = 0; s < NS; ++s ) acc[s][i] = fma( y[1][s], x1, fma( y[0][s], x0, acc[s][i] ) );
             }
         }
         double m[NS][NB];
@@ -218,6 +252,9 @@ template <int CL, int NTM> __global__ void __launch_bounds__( 256, 2 ) k_check_s
 // test and lists.
 template <int CL, bool FIN, int NTM> __global__ void __launch_bounds__( 256, Closure<CL>::NS == 4 ? 1 : 2 ) k_update_small( KParams P ) {
     constexpr int NS = Closure<CL>::NS, NB = ( NTM + LPC - 1 ) / LPC, NF = NS == 4 ? 3 : 2;
+    // nodes at a time, as in the check: two for the cheap fluxes; with three and four
+    // states the registers are short (1-D Euler, 100k cells: 51 us with one, 55 with two)
+    constexpr int KN = NS <= 2 ? 2 : 1;
     const bool finish = FIN && P.finishInUpdate;
     extern __shared__ __align__( 16 ) double smem[];
     if( !P.ctl->active ) return;
@@ -235,6 +272,7 @@ template <int CL, bool FIN, int NTM> __global__ void __launch_bounds__( 256, Clo
         ccount = P.checkCount + ( ( P.ctl->steps + 1 ) & 1 );
     }
     const int stride = gridDim.x * ( blockDim.x / LPC );
+    const bool far   = P.nWork > FAR * stride;
     for( int item0 = ( blockIdx.x * blockDim.x + ( threadIdx.x & ~31 ) ) / LPC; item0 < P.nWork; item0 += stride ) {
         const int item   = item0 + lane / LPC;
         const bool valid = item < P.nWork;
@@ -246,6 +284,16 @@ template <int CL, bool FIN, int NTM> __global__ void __launch_bounds__( 256, Clo
             P.status[cell]  = UQC_CELL_CONVERGED;
             P.iters[cell]   = 0;
             P.finFlag[cell] = 0;
+        }
+        if( far && item + stride < P.nWork ) {
+            const size_t next = size_t( cell ) + stride;
+            prefetch_cell( P.uQ + next * NS * P.nQ, NS * P.nQ, sub );
+            prefetch_cell( P.uRe + next * ldc, ldc, sub );
+            prefetch_line( sub == 0   ? (const void*)( P.nbr + next * NF )
+                           : sub == 1 ? P.unitN + 2 * next * NF
+                           : sub == 2 ? (const void*)( P.scaledN + 2 * next * NF )
+                                      : P.level + next );
+            prefetch_line( sub & 1 ? (const void*)( P.boundary + next ) : P.area + next );
         }
         const int nTj  = P.nTLevel[P.level[cell]];
         const int nMax = __reduce_max_sync( 0xffffffffu, nTj );
@@ -268,30 +316,43 @@ template <int CL, bool FIN, int NTM> __global__ void __launch_bounds__( 256, Clo
                 sn[f][1]        = P.scaledN[2 * at + 1];
                 len[f]          = sqrt( sn[f][0] * sn[f][0] + sn[f][1] * sn[f][1] );
             }
-            for( int k = sub; k < P.nQ; k += LPC ) {
-                double a[NS], gs[NS];
+            for( int k = sub; k < P.nQ; k += KN * LPC ) {
+                const bool two = KN == 2 && k + LPC < P.nQ;
+                const int kk[2] = {k, two ? k + LPC : k};
+                double gs[KN][NS];
 #pragma unroll
-                for( int s = 0; s < NS; ++s ) {
-                    a[s]  = ua[s * P.nQ + k];
-                    gs[s] = 0.0;
+                for( int j = 0; j < KN; ++j ) {
+                    double a[NS];
+#pragma unroll
+                    for( int s = 0; s < NS; ++s ) {
+                        a[s]     = ua[s * P.nQ + kk[j]];
+                        gs[j][s] = 0.0;
+                    }
+                    const typename Problem<CL>::Side sa = Problem<CL>::side( a, P.phys.gamma );
+#pragma unroll
+                    for( int f = 0; f < NF; ++f ) {
+                        double b[NS], y[NS];
+#pragma unroll
+                        for( int s = 0; s < NS; ++s ) b[s] = ub[f][s * P.nQ + kk[j]];
+                        Problem<CL>::flux( a, sa, b, nu[f], sn[f], len[f], y, P.phys );
+#pragma unroll
+                        for( int s = 0; s < NS; ++s ) gs[j][s] += y[s];
+                    }
                 }
-                const typename Problem<CL>::Side sa = Problem<CL>::side( a, P.phys.gamma );
+                if( !two ) {
 #pragma unroll
-                for( int f = 0; f < NF; ++f ) {
-                    double b[NS], y[NS];
-#pragma unroll
-                    for( int s = 0; s < NS; ++s ) b[s] = ub[f][s * P.nQ + k];
-                    Problem<CL>::flux( a, sa, b, nu[f], sn[f], len[f], y, P.phys );
-#pragma unroll
-                    for( int s = 0; s < NS; ++s ) gs[s] += y[s];
+                    for( int s = 0; s < NS && KN == 2; ++s ) gs[KN - 1][s] = 0.0;
                 }
-                const double* row = phiWf + k * P.ld;
+                const double *w0 = phiWf + kk[0] * P.ld, *w1 = phiWf + kk[1] * P.ld;
 #pragma unroll
                 for( int i = 0; i < NTM; ++i ) {
                     if( i >= nMax ) break;
-                    const double w = row[i];
+                    const double x0 = w0[i], x1 = KN == 2 ? w1[i] : 0.0;
 #pragma unroll
-                    for( int s = 0; s < NS; ++s ) acc[s][i] = fma( gs[s], w, acc[s][i] );
+                    for( int s = 0; s < NS; ++s ) {
+                        acc[s][i] = fma( gs[0][s], x0, acc[s][i] );
+                        if( KN == 2 ) acc[s][i] = fma( gs[KN - 1][s], x1, acc[s][i] );
+                    }
                 }
             }
         }
