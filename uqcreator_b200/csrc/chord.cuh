@@ -873,7 +873,8 @@ __host__ __device__ inline size_t sweep_ws_floats( int pairs, int NP ) {
 // warp publishes the two rows in shared memory, one named barrier per pair, and
 // every thread updates its 22 x 3 register block with two FMAs per element. (One
 // pivot at a time, with a barrier, a reciprocal and a publication each: 7190 us for
-// 90,000 cells of 84 duals, pairs 6630; bound by the FMAs of the register block and
+// 90,000 cells of 84 duals, pairs 6630, and 6400 with the four cells' warps of a row
+// group on different schedulers, so that not all publications fall to one; bound by the FMAs of the register block and
 // the shared-memory loads that feed them.) No pivoting: H is symmetric positive definite, and a
 // block that is not (FP32 factor not positive definite) sends the cell to the FP64
 // fallback list.
@@ -885,7 +886,7 @@ template <int CL> __global__ void __launch_bounds__( 512, 1 ) k_invert_sweep( KP
     const int nIn = int( P.ctl->v2Count[round] );
     if( nIn == 0 ) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int cg = warp >> 2, g = warp & 3;    // cell group of the CTA, row group of the warp
+    const int cg = warp >> 2, g = ( warp + cg ) & 3;    // cell group of the CTA, row group of the warp
     const int nT = P.nT, n = NS * nT, pairs = nT * ( nT + 1 ) / 2;
     float* raw  = fsm + size_t( cg ) * sweep_ws_floats( pairs, NP );
     float* prow = raw + sweep_raw_floats( pairs, NP );    // two buffers of two pivot rows (SWEEP_PR floats each)
