@@ -87,6 +87,7 @@ struct uqc_solver {
     int updateNodes = 0, updateLd = 0;    // k_update_mma: nodes per chunk, row stride of its table
     double* d_phiWfP = nullptr;
     void *checkFn = nullptr, *updateFn = nullptr;    // the check kernel, and the update kernel the steps launch
+    bool updateTests = false;    // planned: updateFn tests the next step's convergence
     int* d_activeList = nullptr;    // cells that need Newton: two lists (running step, next step)
     double* d_cellDt  = nullptr;    // per cell: CFL step of its nodal states
     double* d_uRe     = nullptr;    // moments re-projected by the closure epilogue (input of k_update)
@@ -222,7 +223,8 @@ template <class T> T* dupload( const std::vector<T>& v, size_t extra = 0 ) {
     return p;
 }
 
-// Whether k_update tests the next step's convergence (option update_test;
+// Whether k_update is to test the next step's convergence (plan_launches picks the
+// instance and keeps the answer in updateTests, which the steps go by; option update_test,
 // automatic: with a single refinement level. With several, cells whose level
 // flips every step still need the check kernel's epilogue, which then costs
 // as much as testing every cell there).
@@ -309,7 +311,7 @@ KParams make_params( const uqc_solver* h ) {
     P.cellDt       = h->d_cellDt;
     // re-projected moments: a buffer of their own when k_update tests the next
     // step's convergence (it needs them next to u_new), else u itself (in place)
-    P.uRe          = update_test_on( h ) ? h->d_uRe : h->d_u;
+    P.uRe          = h->updateTests ? h->d_uRe : h->d_u;
     P.level        = h->d_level;
     P.nTotalCell   = nullptr;
     P.status       = h->d_status;
@@ -694,7 +696,7 @@ void plan_update_mma( uqc_solver* h, int maxSmem ) {
             if( chunk >= nQ ) return;
             smem = update_mma_doubles( h->nS, nQ, chunk, tiles, warps ) * sizeof( double );
         }
-        void* fn = pick( h->cfg.closure, tiles, update_test_on( h ) ? KERNEL_UPDATE_MMA : KERNEL_UPDATE_MMA_PLAIN );
+        void* fn = pick( h->cfg.closure, tiles, h->updateTests ? KERNEL_UPDATE_MMA : KERNEL_UPDATE_MMA_PLAIN );
         allow_dynamic_smem( fn );
         int occ = 0;
         CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, fn, 32 * warps, smem ) );
@@ -742,7 +744,7 @@ void plan_small( uqc_solver* h ) {
             const int cells = block / LPC;
             grid            = std::min( std::max( 1, occ ) * h->numSMs, std::max( 1, ( h->mesh.nCells + cells - 1 ) / cells ) );
         };
-        if( void* fn = pick_small( cl, ntm, update_test_on( h ) ? KERNEL_UPDATE_SMALL : KERNEL_UPDATE_SMALL_PLAIN ) ) {
+        if( void* fn = pick_small( cl, ntm, h->updateTests ? KERNEL_UPDATE_SMALL : KERNEL_UPDATE_SMALL_PLAIN ) ) {
             h->updateFn   = fn;
             h->updateSmem = table;
             shape( fn, table, h->updateWarpsOpt, h->updateBlock, h->updateGrid );
@@ -814,7 +816,8 @@ void plan_launches( uqc_solver* h ) {
         const size_t perWarp = update_warp_doubles( nS, nQ, h->mesh.nFaces ) * sizeof( double );
         void* kf             = pick( cl, h->group, update_kernel_id( h, true ) );
         void* kp             = pick( cl, h->group, update_kernel_id( h, false ) );
-        void* ku             = update_test_on( h ) ? kf : kp;    // the variant the steps launch
+        h->updateTests       = update_test_on( h );
+        void* ku             = h->updateTests ? kf : kp;    // the variant the steps launch
         h->updateFn          = ku;
         allow_dynamic_smem( kf );
         allow_dynamic_smem( kp );
@@ -1225,12 +1228,12 @@ void enqueue_closure_phase( uqc_solver* h, KParams P, bool check = true ) {
 
 void enqueue_update( uqc_solver* h, KParams P ) {
     step_lists( h, P );
-    P.finishInUpdate = update_test_on( h );
+    P.finishInUpdate = h->updateTests;
     void* args[]     = {&P};
     launch( h, h->updateFn, h->updateGrid, h->updateBlock, h->updateSmem, args );
 }
 
-bool check_after_update( const uqc_solver* h ) { return !( update_test_on( h ) && h->tab.nLevels == 1 ); }
+bool check_after_update( const uqc_solver* h ) { return !( h->updateTests && h->tab.nLevels == 1 ); }
 
 // n time steps
 void enqueue_steps( uqc_solver* h, KParams& P, int n ) {
@@ -1601,6 +1604,14 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
     h->cfg.newtonMode    = newton_mode;
     ++h->planGen;
     return guarded( h, [&] {
+        if( h->deviceReady ) {
+            // the update's instance (with or without the next step's test) and the mixed
+            // form's rounds depend on the Newton mode and the iteration limit
+            const int form = h->v2Mode;
+            plan_launches( h );
+            // the held factors' format depends on the form
+            if( h->v2Mode != form && h->precision == UQC_MIXED && h->chord && !h->mixedNewton ) reset_factor_store( h );
+        }
         invalidate_lists( h );    // the next step's list was built with the old test
         return UQC_OK;
     } );
@@ -2362,7 +2373,7 @@ int uqc_step_host( uqc_solver* h, const double* u_in, const double* lambda_in, c
         {
             KParams U = P;
             step_lists( h, U );
-            U.finishInUpdate = update_test_on( h );
+            U.finishInUpdate = h->updateTests;
             U.blockPartial   = h->d_chunkPartial;
             U.updChunks      = CHUNKS;
             void* ku         = h->updateFn;
