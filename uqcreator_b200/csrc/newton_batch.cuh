@@ -141,28 +141,32 @@ __device__ __forceinline__ void acc_to_b( double c0, double c1, int lane, double
 // is (the back substitution reads it). Warp 0 takes the next diagonal tile
 // alone, and its inverse, which is the dependent chain of the step; the last
 // warp takes the right-hand side. Returns false if a pivot block is not
-// positive definite (posv's info > 0). flag: one int in shared memory, zero
-// on entry. Warp 0 of every slot issues on the same scheduler (slots are a
-// multiple of four warps apart), where its chain does not queue behind the
-// other warps' products on the FP64 pipe.
+// positive definite (posv's info > 0). flag: two ints in shared memory, zero
+// on entry, for the diagonal tiles of even and odd columns: step J's warps read
+// tile J's after the step's barrier while warp 0 may already be writing tile
+// J + 1's, and tile J + 2's is written only after the next barrier, which every
+// reader of tile J's has reached. (With one flag for all, a warp that read it late
+// could leave a step, and a barrier, before the others.) Warp 0 of every slot
+// issues on the same scheduler (slots are a multiple of four warps apart), where
+// its chain does not queue behind the other warps' products on the FP64 pipe.
 template <int GROUP> __device__ bool eliminate_slot( const Grp<GROUP>& g, double* H, int nb, int* flag ) {
     constexpr int G = GROUP / 32;
     const int warp = g.r >> 5, lane = g.r & 31, gr = lane >> 2, t = lane & 3;
     const int o  = rix( gr, 2 * t );                         // accumulator place in a tile (16 bytes)
     const int f0 = rix( t, gr ), f1 = rix( t + 4, gr );      // fragment places
     double* rhs = H + hrhs( nb );
-    auto invert = [&]( double* D, double c0, double c1 ) {
-        if( !tile_sweep_inverse( D, c0, c1, lane ) && lane == 0 ) *flag = 1;
+    auto invert = [&]( int J, double* D, double c0, double c1 ) {
+        if( !tile_sweep_inverse( D, c0, c1, lane ) && lane == 0 ) flag[J & 1] = 1;
     };
     if( warp == 0 ) {
         // the first tile: only its upper half is filled
         const double c0 = H[gr <= 2 * t ? o : rix( 2 * t, gr )], c1 = H[gr <= 2 * t + 1 ? o + 1 : rix( 2 * t + 1, gr )];
         __syncwarp();
-        invert( H, c0, c1 );
+        invert( 0, H, c0, c1 );
     }
     for( int J = 0; J + 1 < nb; ++J ) {
         g.sync();    // the diagonal tile's inverse and all of row J's updates are in place
-        if( *flag ) return false;
+        if( flag[J & 1] ) return false;
         const int K     = J + 1;
         const double* N = H + htile( J, J );
         const double n0 = N[f0], n1 = N[f1];    // symmetric: also the A fragments
@@ -184,7 +188,7 @@ template <int GROUP> __device__ bool eliminate_slot( const Grp<GROUP>& g, double
             __syncwarp();
             dmma_8x8x4( c0, c1, A[f0], b0 );
             dmma_8x8x4( c0, c1, A[f1], b1 );
-            invert( D, c0, c1 );
+            invert( K, D, c0, c1 );
         }
         if( G == 1 || warp > 0 ) {
             const int worker = G == 1 ? 0 : warp - 1, workers = G == 1 ? 1 : G - 1;
@@ -252,7 +256,7 @@ template <int GROUP> __device__ bool eliminate_slot( const Grp<GROUP>& g, double
         }
     }
     g.sync();
-    return !*flag;
+    return !flag[( nb - 1 ) & 1];
 }
 
 // x = H^-1 b by one warp from eliminate_slot's tiles: x_J = -N_JJ b_J, then every
@@ -329,7 +333,7 @@ __global__ void __launch_bounds__( 32 * W, CTAS ) k_newton( KParams P, int mode 
     double *lam = ws + S.lam, *lamI = ws + S.lamI, *uh = ws + S.uh, *ms = ws + S.m, *dir = ws + S.d, *uk = ws + S.uk, *red = ws + S.red;
     double* H        = ws + S.hd;    // Hessian tiles; between iterations DU and the partial sums
     double* part     = H + NP * S.duStride;
-    int* flag        = reinterpret_cast<int*>( red + 24 );
+    int* flag        = reinterpret_cast<int*>( red + 24 );    // two
     const size_t ldc = size_t( NS ) * P.nT;
     const int nQ4    = ( P.nQ + 3 ) & ~3;
     const double eps = P.eps;
@@ -606,7 +610,7 @@ __global__ void __launch_bounds__( 32 * W, CTAS ) k_newton( KParams P, int mode 
                 const int s = idx / nTj, i = idx - s * nTj;
                 H[hrhs( nb ) + idx] = idx < n ? ms[s * P.nT + i] - uh[s * P.nT + i] : 0.0;
             }
-            if( g.r == 0 ) *flag = 0;
+            if( g.r == 0 ) flag[0] = flag[1] = 0;
         }
         __syncthreads();
         PT_END( tScatter, 28 );
