@@ -55,3 +55,22 @@ def test_statuses_and_neighbours(name):
     alone, status = s.closure_solve_host(lam[~bad], u[~bad])
     assert not status.any()
     np.testing.assert_array_equal(got[~bad], alone)
+
+
+@pytest.mark.parametrize("newton,group", [("reference", 256), ("guarded", 256), ("safe", 64), ("safe", 256)])
+@pytest.mark.parametrize("name", ["sw_24", "euler_84"])
+def test_general_kernel(name, newton, group):
+    """The same through the general kernel's Cholesky, two and eight warps a cell."""
+    toml = CASES[name]
+    toml = toml.replace('newton = "guarded"', 'newton = "reference"').replace('newton = "reference"', f'newton = "{newton}"')
+    o, u, lam, bad = _batch(toml, 46)
+    _, expect, _ = o.solve_closure(lam, u)
+    np.testing.assert_array_equal(expect, np.where(bad, NOT_PD, 0))
+    s = Solver(toml)
+    s.set_option("closure_group", group)
+    got, status = s.closure_solve_host(lam, u)
+    np.testing.assert_array_equal(status, expect)
+    np.testing.assert_array_equal(got[bad], lam[bad])
+    alone, status = s.closure_solve_host(lam[~bad], u[~bad])
+    assert not status.any()
+    np.testing.assert_array_equal(got[~bad], alone)

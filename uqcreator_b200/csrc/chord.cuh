@@ -764,7 +764,7 @@ template <int CL, bool RAW> __global__ void __launch_bounds__( 256, 1 ) k_invert
     float* Iv         = D + a16( size_t( hnb( nMax ) ) * 8 * 4 ) / 4;
     float* X          = Iv + a16( size_t( hnb( nMax ) ) * 8 * 4 ) / 4;
     int* flag         = reinterpret_cast<int*>( X + a16( size_t( xpacked( nMax ) ) * 4 ) / 4 );
-    int* itemS        = flag + 1;
+    int* itemS        = flag + 2;    // cholesky_la has two flags
     float* du         = reinterpret_cast<float*>( flag + 16 );
     double* LA        = reinterpret_cast<double*>( reinterpret_cast<unsigned char*>( du ) + a16( size_t( ( NP + 1 ) & ~1 ) * P.nQ * 4 ) );
     for( ;; ) {

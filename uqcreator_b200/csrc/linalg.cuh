@@ -359,25 +359,29 @@ template <class T> __device__ __forceinline__ void rhs_update( T* H, int J, int 
 // U(j,j), I[j] = 1/U(j,j) (padded to 8 nb entries), and the strictly lower
 // half of each diagonal tile holds the transposed inverse of its U block.
 // Returns 0, or j + 1 for the first pivot that is not positive (posv's
-// info > 0). flag: one int in shared memory.
+// info > 0). flag: two ints in shared memory, for the tiles of even and odd
+// columns: a warp reads tile K's after step J's barrier, when warp 0 may already
+// be factoring tile K + 1; tile K + 2's write waits for the next barrier, which
+// every reader of tile K's has reached.
 template <int GROUP, class T>
 __device__ int cholesky_la( const Grp<GROUP>& g, T* H, int n, T* D, T* I, int* flag ) {
     constexpr int W = GROUP / 32;
     const int nb = hnb( n ), warp = g.r >> 5, lane = g.r & 31;
     if( warp == 0 ) {
         if( lane == 0 ) {
-            *flag = 0;
+            flag[0] = flag[1] = 0;
             tile_factor<T>( H, D, I, 0, flag );
         }
         __syncwarp();
         tile_inverse<T>( H, I, 0, lane );
         __syncwarp();
-        if( !*flag ) tile_row_solve_mma<T>( H, 0, nb, I, lane );
+        if( !flag[0] ) tile_row_solve_mma<T>( H, 0, nb, I, lane );
     }
     g.sync();
-    if( *flag ) return *flag;
+    if( flag[0] ) return flag[0];
     for( int J = 0; J + 1 < nb; ++J ) {
         const int K = J + 1;
+        int* bad    = flag + ( K & 1 );
         CT_BEGIN( tc );
         if( warp == 0 ) {
             CT_BEGIN( t0 );
@@ -386,7 +390,7 @@ __device__ int cholesky_la( const Grp<GROUP>& g, T* H, int n, T* D, T* I, int* f
             __syncwarp();
             CT_END( t0, 14, g.r == 0 );
             CT_BEGIN( t1 );
-            if( lane == 0 ) tile_factor<T>( H + htile( K, K ), D, I, K * 8, flag );
+            if( lane == 0 ) tile_factor<T>( H + htile( K, K ), D, I, K * 8, bad );
             __syncwarp();
             CT_END( t1, 12, g.r == 0 );
             CT_BEGIN( t2 );
@@ -394,7 +398,7 @@ __device__ int cholesky_la( const Grp<GROUP>& g, T* H, int n, T* D, T* I, int* f
             __syncwarp();
             CT_END( t2, 13, g.r == 0 );
             CT_BEGIN( t3 );
-            if( !*flag ) tile_row_solve_mma<T>( H, K, nb, I, lane );
+            if( !*bad ) tile_row_solve_mma<T>( H, K, nb, I, lane );
             CT_END( t3, 15, g.r == 0 );
         }
         CT_END( tc, 8, g.r == 0 );
@@ -414,7 +418,7 @@ __device__ int cholesky_la( const Grp<GROUP>& g, T* H, int n, T* D, T* I, int* f
         g.sync();
         CT_END( tb, 10, g.r == 0 );
         CT_END( tb, 11, g.r == 32 );
-        if( *flag ) return *flag;
+        if( *bad ) return *bad;
     }
     return 0;
 }
