@@ -146,3 +146,33 @@ def test_rounds_are_reproducible_and_keep_inverses():
     ub = s.download_state()[0]
     assert a["newton_iterations"] == b["newton_iterations"]
     np.testing.assert_array_equal(ua, ub)
+
+
+@pytest.mark.parametrize("degree", [1, 2])
+@pytest.mark.parametrize("options", [{"mixed_hessian": 1}, {"mixed_hessian": 2}, {"mixed_max_iterations": 50}, {"closure_group": 32},
+                                     {"closure_group": 256}], ids=lambda o: "_".join(f"{k}_{v}" for k, v in o.items()))
+def test_rounds_of_few_moments(degree, options):
+    """Up to 6 moments the several-lanes update kernel lists the cells for the
+    rounds, with the gradient they start from: the oracle's moments, and the
+    Newton work of the check kernel's lists (update_test 0; the two gradients
+    differ by rounding, which moves an iteration count in one cell of 10^5)."""
+    toml = W.euler2d(nx=24, ny=5, degree=degree, nquad=4)
+    o = Oracle(toml, W.mesh_for(toml))
+    o.init_state()
+    o.step(5)
+    uo = o.get_state()[0]
+    info = []
+    for test in (1, 0):
+        s = Solver(toml)
+        s.set_precision(MIXED)
+        for k, v in options.items():
+            s.set_option(k, v)
+        s.set_option("update_test", test)
+        assert s.form()["mixed_form"] == options.get("mixed_hessian", 2)
+        s.init_state()
+        info.append(s.step(5))
+        assert info[-1]["failed_cells"] == 0 and info[-1]["steps"] == 5
+        us = s.download_state()[0]
+        assert float(np.abs(us - uo).sum() / np.abs(uo).sum()) <= 1e-6
+    assert info[0]["fallback_cells"] == info[1]["fallback_cells"]
+    assert abs(info[0]["newton_iterations"] - info[1]["newton_iterations"]) <= 0.01 * info[1]["newton_iterations"]

@@ -391,6 +391,20 @@ template <int CL, bool FIN, int NTM> __global__ void __launch_bounds__( 256, Clo
                 fin = pass && !fixed && level_rule( P, level_indicator( P, [&]( int i ) { return u[i]; }, lev, nTj ), lev ) == lev;
             }
             if( fin && sub == 0 ) finish_cell( P, cell, u0, dtNext );
+            if constexpr( NS == 4 ) {
+                // the gradient the mixed form's rounds start from (see test_next_step),
+                // from the lane's own moments
+                if( P.gStore && valid && !pass ) {
+                    double* gs = P.gStore + size_t( cell ) * P.gStride;
+                    for( int i = sub; i < nTj; i += LPC )
+#pragma unroll
+                        for( int s = 0; s < NS; ++s ) {
+                            const size_t at  = size_t( cell ) * ldc + s * P.nT + i;
+                            gs[s * nTj + i]  = P.uRe[at] - P.u[at];
+                        }
+                    if( sub == 0 ) gs[ldc] = sqrt( sq );
+                }
+            }
             warp_append( pass && !fin && sub == 0, cell, clist, ccount, lane );
             warp_append( valid && !pass && sub == 0, cell, nlist, ncount, lane );
         }
