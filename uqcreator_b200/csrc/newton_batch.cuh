@@ -87,7 +87,7 @@ __host__ __device__ inline int newton_chunk( int nS, int nT, int nQ ) {
     return fit < 4 ? 0 : fit - ( fit + 4 ) % 8;
 }
 
-// D <- -T^-1 for a symmetric positive definite 8 x 8 tile T held as an mma
+// T <- -T^-1 for a symmetric positive definite 8 x 8 tile T held as an mma
 // accumulator (lane 4 g + t: c0, c1 = row g, columns 2t and 2t + 1), by sweeps on
 // the four 2 x 2 pivot blocks P (rows and columns p): A_pp -> -P^-1, A_rp -> A_rp
 // P^-1, A_rc -> A_rc - A_rp P^-1 A_pc. With P^-1 = adj(P) / det(P) the products with
@@ -96,8 +96,8 @@ __host__ __device__ inline int newton_chunk( int nS, int nT, int nQ ) {
 // 820 cycles for the tile on an idle SM, against 1,020 for its element-wise
 // Cholesky factor and triangular inverse in every lane's registers. This is the
 // elimination's dependent chain. Returns false if a leading minor is not
-// positive.
-__device__ __forceinline__ bool tile_sweep_inverse( double* D, double c0, double c1, int lane ) {
+// positive, or a block's determinant not within 2^+-1000.
+__device__ __forceinline__ bool tile_sweep( double& c0, double& c1, int lane ) {
     const unsigned full = 0xffffffffu;
     const int g = lane >> 2, t = lane & 3;
     bool ok = true;
@@ -108,7 +108,9 @@ __device__ __forceinline__ bool tile_sweep_inverse( double* D, double c0, double
         const double v00 = __shfl_sync( full, c0, 8 * p + t ), v01 = __shfl_sync( full, c1, 8 * p + t );
         const double v10 = __shfl_sync( full, c0, 8 * p + 4 + t ), v11 = __shfl_sync( full, c1, 8 * p + 4 + t );
         const double det = fma( a, d, -b * b );
-        ok               = ok && a > 0.0 && det > 0.0;
+        // a > 0 and 2^-1000 <= det < 2^1000 by the high words (beside the FP64 pipe; a NaN is
+        // out of range)
+        ok             = ok && __double2hiint( a ) > 0 && unsigned( __double2hiint( det ) - 0x01700000 ) < 0x7D000000u;
         const double r   = reciprocal( det );
         // A_rp adj(P); the pivot rows take -adj(P)
         const bool inRow = ( g >> 1 ) == p, inCol = t == p;
@@ -119,8 +121,32 @@ __device__ __forceinline__ bool tile_sweep_inverse( double* D, double c0, double
         c0               = fma( -s0, r, inRow || inCol ? 0.0 : c0 );
         c1               = fma( -s1, r, inRow || inCol ? 0.0 : c1 );
     }
-    *reinterpret_cast<double2*>( D + rix( g, 2 * t ) ) = make_double2( c0, c1 );
     return ok;
+}
+
+// The sweep of S T S, S the powers of two that take T's diagonal entries to [1, 4):
+// the determinants of entries beyond 2^+-500 leave the format's range (or the
+// reciprocal's) although the entries do not. D <- -S (S T S)^-1 S.
+static __device__ __noinline__ bool tile_sweep_scaled( double* D, double c0, double c1, int lane ) {
+    const unsigned full = 0xffffffffu;
+    const int g = lane >> 2, t = lane & 3;
+    const double diag = ( g & 1 ) ? c1 : c0;    // of row g, in the lane that holds its column
+    const double dg = __shfl_sync( full, diag, 4 * g + ( g >> 1 ) ), d0 = __shfl_sync( full, diag, 9 * t ), d1 = __shfl_sync( full, diag, 9 * t + 4 );
+    if( __any_sync( full, !( dg > 0.0 ) || !isfinite( dg ) ) ) return false;
+    const int e = -( ilogb( dg ) >> 1 ), e0 = e - ( ilogb( d0 ) >> 1 ), e1 = e - ( ilogb( d1 ) >> 1 );
+    c0            = scalbn( c0, e0 );
+    c1            = scalbn( c1, e1 );
+    const bool ok = tile_sweep( c0, c1, lane );
+    *reinterpret_cast<double2*>( D + rix( g, 2 * t ) ) = make_double2( scalbn( c0, e0 ), scalbn( c1, e1 ) );
+    return ok;
+}
+
+// D <- -T^-1 (see tile_sweep); returns false if T is not positive definite.
+__device__ __forceinline__ bool tile_sweep_inverse( double* D, double c0, double c1, int lane ) {
+    double x0 = c0, x1 = c1;
+    if( !tile_sweep( x0, x1, lane ) ) return tile_sweep_scaled( D, c0, c1, lane );
+    *reinterpret_cast<double2*>( D + rix( lane >> 2, 2 * ( lane & 3 ) ) ) = make_double2( x0, x1 );
+    return true;
 }
 
 // B fragments (rows t and t + 4 of column g) of a tile held as an accumulator.
