@@ -3,7 +3,7 @@ range although the entries do not (a state's unit is the user's)."""
 import numpy as np
 import pytest
 
-from uqcreator_b200 import workloads as W
+from uqcreator_b200 import MIXED, workloads as W
 from uqcreator_b200.solver import Solver
 
 pytestmark = pytest.mark.gpu
@@ -30,3 +30,28 @@ def test_batched_newton(degree, newton):
     big, status = solver(2.0 ** 512).closure_solve_host(np.zeros_like(u), u * 2.0 ** 512)
     assert not status.any()
     np.testing.assert_array_equal(big, lam)
+
+
+def test_mixed_inverse():
+    """Pressure in a unit that takes the energy block beyond 1e19, whose square
+    FP32 does not hold: the inverse is not formed, and the cells take the FP64
+    form's iterations, no others."""
+    unit, text = 2.0 ** 40, W.euler2d(nx=12, ny=4)
+    s = Solver(text)
+    s.init_state()
+    s.step(2)
+    u, lam, level = s.download_state()
+    r = np.sqrt(unit)
+    u = u * np.array([1.0, r, r, unit])[:, None]
+    lam = lam / np.array([1.0, r, r, unit])[:, None]
+    lam[:, 0, 0] -= np.log(unit)
+    info = []
+    for precision in (0, MIXED):
+        s = Solver(W.euler2d(nx=12, ny=4, eps=1e-10 * unit))
+        s.set_precision(precision)
+        s.upload_state(u, lam, level)
+        info.append(s.step(1))
+        assert info[-1]["failed_cells"] == 0
+    assert info[0]["newton_iterations"] > 0
+    assert info[1]["newton_iterations"] == info[0]["newton_iterations"]
+    assert info[1]["fallback_cells"] > 0
