@@ -107,3 +107,21 @@ def test_chord_newton_reuses_factors_reproducibly():
     c = s.step(4)
     assert _moment_err(s.download_state()[0], ref.download_state()[0]) <= TOL
     assert c["newton_iterations"] <= a["newton_iterations"]
+
+
+@pytest.mark.parametrize("n", [40, 400])
+def test_batch_larger_than_the_mesh(n):
+    """A closure-only batch of more cells than the mesh has, all of them handed
+    to the FP64 form after two iterations: the list of those cells is the batch's."""
+    toml = W.burgers1d(ncells=3, degree=11, nquad=24)
+    a, b = Solver(toml), Solver(toml)
+    b.set_precision(MIXED)
+    b.set_option("mixed_max_iterations", 2)
+    _, phi_wf, xi, _ = a.tables()
+    r = np.random.default_rng(4)
+    u = (7.5 + 2 * r.uniform(-1, 1, (n, 1)) + r.uniform(-1, 1, (n, 1)) * xi[:, 0])[:, None, :] @ phi_wf
+    la, sa = a.closure_solve_host(np.zeros_like(u), u)
+    lb, sb = b.closure_solve_host(np.zeros_like(u), u)
+    assert not sa.any() and not sb.any()
+    # eps over the smallest eigenvalue of the Hessians (states in [4.5, 10.5]: DU above 1.5)
+    np.testing.assert_allclose(lb, la, rtol=0, atol=2 * 1e-10 / 1.5)

@@ -79,6 +79,8 @@ struct uqc_solver {
     unsigned* d_xNt = nullptr;
     int *d_xStatus = nullptr, *d_xIters = nullptr;
     size_t xCap = 0;
+    int* d_xFallback = nullptr;    // the mixed form's fallback list of a batch larger than the mesh
+    size_t xFallbackCap = 0;
     void* h_batch = nullptr;    // uqc_closure_solve_host: pinned memory of a few cells' batch (HOST_BATCH_BYTES)
     // launch shapes
     int closureBlock = 256, closureGrid = 0, updateBlock = 256, updateGrid = 0, auxGrid = 0, auxBlock = 256;
@@ -1097,7 +1099,7 @@ void release( uqc_solver* h ) {
                     (void*)h->d_unitN, (void*)h->d_scaledN, (void*)h->d_nbr, (void*)h->d_boundary, (void*)h->d_u, (void*)h->d_lam,
                     (void*)h->d_bndNormal, (void*)h->d_uQ, (void*)h->d_uOld0, (void*)h->d_blockPartial, (void*)h->d_chunkPartial, (void*)h->d_level, (void*)h->d_status,
                     (void*)h->d_iters, (void*)h->d_ctl, (void*)h->d_xLam, (void*)h->d_xU, (void*)h->d_xNt, (void*)h->d_xStatus,
-                    (void*)h->d_xIters, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_phiT, (void*)h->d_pairSlots, (void*)h->d_tinyTab, (void*)h->d_phiWfP, (void*)h->d_fallbackList,
+                    (void*)h->d_xIters, (void*)h->d_xFallback, (void*)h->d_activeList, (void*)h->d_cellDt, (void*)h->d_uRe, (void*)h->d_checkList, (void*)h->d_finFlag, (void*)h->d_phiF, (void*)h->d_phiT, (void*)h->d_pairSlots, (void*)h->d_tinyTab, (void*)h->d_phiWfP, (void*)h->d_fallbackList,
                     (void*)h->d_factorStore, (void*)h->d_factorLevel, (void*)h->d_gStore, (void*)h->d_v2Lists,
                     (void*)h->d_chordIters, (void*)h->d_qTiles, (void*)h->d_sendCells, (void*)h->d_filter, (void*)h->d_lassoParam,
                     (void*)h->d_lassoL1} )
@@ -1163,7 +1165,7 @@ void launch_closure( uqc_solver* h, KParams& P, int mode ) {
             launch( h, pick( cl, 32, KERNEL_CHORD ), h->chordGrid, h->chordBlock, h->chordSmem, args );
         }
         KParams F      = P;
-        F.activeList   = h->d_fallbackList;
+        F.activeList   = P.fallbackList;
         F.activeCount  = &h->d_ctl->nFallback;
         F.listParity   = 0;
         F.workCounter  = &h->d_ctl->workCounter2;
@@ -1178,7 +1180,7 @@ void launch_closure( uqc_solver* h, KParams& P, int mode ) {
         void* margs[]  = {&M, &mode};
         launch( h, pick( h->cfg.closure, h->mixedGroup, 4 ), h->mixedGrid, h->mixedBlock, h->mixedSmem, margs );
         KParams F     = P;
-        F.activeList  = h->d_fallbackList;
+        F.activeList  = P.fallbackList;
         F.activeCount = &h->d_ctl->nFallback;
         F.listParity  = 0;    // one fallback list
         F.workCounter = &h->d_ctl->workCounter2;
@@ -2160,6 +2162,7 @@ int uqc_solve_closure( uqc_solver* h, uqc_step_info* info ) {
 }
 
 void ensure_scratch( uqc_solver* h, size_t n );
+static void fit_fallback_list( uqc_solver* h, KParams& P, size_t n );
 int uqc_solve_closure_cells( uqc_solver* h, const unsigned* cells, int n_cells, double tol, int max_iter, uqc_step_info* info ) {
     if( !h || n_cells < 0 || ( cells && n_cells == 0 ) || tol < 0.0 || max_iter < 0 ) return UQC_ERR_ARGUMENT;
     if( !h->stateReady ) return fail( h, UQC_ERR_STATE, "no state" );
@@ -2186,6 +2189,7 @@ int uqc_solve_closure_cells( uqc_solver* h, const unsigned* cells, int n_cells, 
             P.activeList  = list;
             P.activeCount = cnt;
             P.listParity  = 0;
+            fit_fallback_list( h, P, size_t( n_cells ) );
         }
         launch_closure( h, P, 0 );
         CK( cudaGetLastError() );
@@ -2465,6 +2469,20 @@ void ensure_scratch( uqc_solver* h, size_t n ) {
     h->xCap      = n;
 }
 
+// A closure-only batch of n cells may hand all of them to the FP64 form: beyond
+// the mesh's cells the list of the time steps is too short.
+static void fit_fallback_list( uqc_solver* h, KParams& P, size_t n ) {
+    if( h->precision != UQC_MIXED || n <= size_t( h->mesh.nCells ) ) return;
+    if( n > h->xFallbackCap ) {
+        if( h->d_xFallback ) cudaFree( h->d_xFallback );
+        h->d_xFallback  = nullptr;
+        h->xFallbackCap = 0;
+        h->d_xFallback  = dalloc<int>( n );
+        h->xFallbackCap = n;
+    }
+    P.fallbackList = h->d_xFallback;
+}
+
 static void closure_on( uqc_solver* h, int n, double* d_lam, const double* d_u, const unsigned* d_nt, int* d_status, int* d_iters ) {
     KParams P     = make_params( h );
     P.nCells      = n;
@@ -2475,6 +2493,7 @@ static void closure_on( uqc_solver* h, int n, double* d_lam, const double* d_u, 
     P.nTotalCell  = d_nt;
     P.status      = d_status;
     P.iters       = d_iters;
+    fit_fallback_list( h, P, size_t( n ) );
     reset_work( h );
     launch_closure( h, P, 0 );
     CK( cudaGetLastError() );
