@@ -1,9 +1,11 @@
 """Autotuner of the time step's launch shapes and schedules.
 
 What it chooses, per configuration shape:
-- closure (FP64 form): a cell on one warp, two warps (several cells per CTA,
-  named barriers) or a whole CTA, with the basis tables staged in shared memory
-  or read through L1 (which leaves room for more cells per SM);
+- closure (FP64 form): a cell on one warp (32; the kernel of tiny systems where it
+  applies), the batched kernel whose cells iterate together where its shapes
+  fit, else two warps a cell (64), or a whole CTA (256), with the basis tables
+  staged in shared memory or read through L1 (which leaves room for more cells
+  per SM);
 - chord schedule of the single mixed kernel: theta and whether the held FP32
   factor is kept as its packed inverse;
 - chord schedule (mixed form in rounds, 2-D Euler): theta, the contraction
@@ -76,7 +78,9 @@ def groups(n_per_cell: int, mixed_form: int = 0, mixed: bool = False):
 
 
 def _key(solver, precision, mixed_form):
-    return (f"v4_s{solver.n_states}_t{solver.n_total}_q{solver.n_quad}_l{solver.n_levels}_d{solver.dim_xi}_p{precision}"
+    # the version goes up when an option's meaning does (v5: closure_group 32 and
+    # 256 exclude the batched Newton kernel)
+    return (f"v5_s{solver.n_states}_t{solver.n_total}_q{solver.n_quad}_l{solver.n_levels}_d{solver.dim_xi}_p{precision}"
             f"_m{mixed_form if precision else 0}")
 
 
