@@ -1323,10 +1323,20 @@ unsigned long long factor_store_bytes( const uqc_solver* h );
 unsigned long long device_bytes_of( const uqc_solver* h ) {
     const unsigned long long N = (unsigned long long)h->mesh.nCells, F = (unsigned long long)h->mesh.nFaces;
     const unsigned long long ldc = h->ldc, sq = (unsigned long long)h->nS * h->tab.nQ;
-    const unsigned long long tab = ( (unsigned long long)h->tab.nQ * h->ld + 8 ) * ( 8 + 8 + 4 ) + h->tab.xi.size() * 8 + h->tab.nQ * 8;
+    const unsigned long long nT = (unsigned long long)h->tab.nT, nQ4 = (unsigned long long)( ( h->tab.nQ + 3 ) & ~3 );
+    unsigned long long tab      = ( (unsigned long long)h->tab.nQ * h->ld + 8 ) * ( 8 + 8 + 4 ) + h->tab.xi.size() * 8 + h->tab.nQ * 8 + nT * nQ4 * 8;
+    if( !closure_linear( h->cfg.closure ) ) tab += nT * ( nT + 1 ) / 2 * closure_np( h->cfg.closure ) * 4;    // k_newton's pair places
+    if( h->ldc <= size_t( SMALL_N ) && h->tab.nQ <= TINY_MAX_NODES )
+        tab += (unsigned long long)tiny_cols( h->ldc <= size_t( TINY_N ) ? TINY_N : SMALL_N ) * h->tab.nQ * 8;
+    if( h->cfg.closure == 1 )
+        for( int tiles : UPD_TILES )
+            if( nT <= 8ull * tiles ) {
+                tab += nQ4 * upd_ld( tiles ) * 8;    // k_update_mma's table
+                break;
+            }
     const unsigned long long d8  = N * ( 3 * ldc + 1 + 1 + 1 + 2 + 4 * F ) + ( N + 1 ) * sq;    // state (u, re-projected u, lambda), uQ, geometry, cell dt
     const unsigned long long d4  = N * ( F + 1 + 1 + 1 + 1 + 2 + 2 + 1 );                     // nbr, boundary, level, status, iters, lists
-    return tab + 8 * d8 + 4 * d4 + N + ( mesh_has_walls( h->mesh ) ? 16 * N : 0 ) + sizeof( Control ) + 8 * 4096 + 
+    return tab + 8 * d8 + 4 * d4 + N + ( mesh_has_walls( h->mesh ) ? 16 * N : 0 ) + sizeof( Control ) + 8 * 4096 +
            // (counted before the device side is set up even where the default then runs without the store)
            ( h->precision == UQC_MIXED && h->chord && !( h->deviceReady && !h->d_factorStore ) ? factor_store_bytes( h ) : 0 );
 }
