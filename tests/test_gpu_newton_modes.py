@@ -74,3 +74,26 @@ def test_mixed_form_follows_the_mode():
     s.init_state()
     assert s.step(STEPS)["failed_cells"] == 0
     np.testing.assert_allclose(s.download_state()[0], expect, rtol=0, atol=1e-6 * np.abs(expect).max())
+
+
+def test_rounds_that_appear_between_steps():
+    """mixed_chord 0 and 1 again on a live handle: the rounds start from gradients
+    that the single kernel's steps did not store, so every cell is tested anew.
+    The same state uploaded again, where every cell is, gives the same steps."""
+    s = Solver(W.euler2d(nx=24, ny=5, tend=10.0))
+    s.set_precision(MIXED)
+    s.init_state()
+    s.set_option("mixed_chord", 0)
+    s.step(2)
+    state, t = s.download_state(), s.step(0)["t"]
+    s.set_option("mixed_chord", 1)
+    assert s.form()["mixed_form"] == 2
+    a = s.step(STEPS)
+    ua, la, _ = s.download_state()
+    s.upload_state(*state, t=t)
+    b = s.step(STEPS)
+    ub, lb, _ = s.download_state()
+    assert a["failed_cells"] == b["failed_cells"] == 0
+    assert a["fallback_cells"] == b["fallback_cells"] and a["newton_iterations"] == b["newton_iterations"]
+    np.testing.assert_array_equal(ua, ub)
+    np.testing.assert_array_equal(la, lb)

@@ -880,6 +880,8 @@ void plan_launches( uqc_solver* h ) {
     plan_update_mma( h, maxSmem );
     plan_small( h );
     plan_newton( h, maxSmem );
+    const int wasForm  = h->v2Mode;
+    const bool wasFp64 = h->mixedNewton, wasInverse = h->chordInverse;
     plan_mixed( h, maxSmem );
     plan_rounds( h, maxSmem );
     // Which kernel the mixed form's default runs on the 2-D Euler closure. Steps:
@@ -891,11 +893,11 @@ void plan_launches( uqc_solver* h ) {
     // 430 and, on 200k cells, 1460 / 5080; without rounds: 80 duals, 216 nodes 968
     // / 801; 140 duals, 512 nodes 4553 / 3816 (first step 34193 / 17540). Any option
     // that asks for the mixed kernels' form keeps them.
-    const bool was     = h->mixedNewton;
     h->mixedNewtonOnce = h->newtonId && h->mixedOk && h->roundsOpt == -1 && h->chord && h->mixedMaxIter == 0;
     h->mixedNewton     = h->mixedNewtonOnce && ( h->v2Mode == 0 || n <= 48 );
-    if( h->deviceReady && h->precision == UQC_MIXED && was != h->mixedNewton ) {
-        // the mixed kernels need their store, and a next-step list with gradients
+    if( h->deviceReady && h->precision == UQC_MIXED && ( wasForm != h->v2Mode || wasFp64 != h->mixedNewton || wasInverse != h->chordInverse ) ) {
+        // another form: a store of its format, empty, and for the rounds a next-step
+        // list with gradients
         if( h->chord && !h->mixedNewton ) reset_factor_store( h );
         invalidate_lists( h );
     }
@@ -1616,14 +1618,9 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
     h->cfg.newtonMode    = newton_mode;
     ++h->planGen;
     return guarded( h, [&] {
-        if( h->deviceReady ) {
-            // the update's instance (with or without the next step's test) and the mixed
-            // form's rounds depend on the Newton mode and the iteration limit
-            const int form = h->v2Mode;
-            plan_launches( h );
-            // the held factors' format depends on the form
-            if( h->v2Mode != form && h->precision == UQC_MIXED && h->chord && !h->mixedNewton ) reset_factor_store( h );
-        }
+        // the update's instance (with or without the next step's test) and the mixed form's
+        // rounds depend on the Newton mode and the iteration limit
+        if( h->deviceReady ) plan_launches( h );
         invalidate_lists( h );    // the next step's list was built with the old test
         return UQC_OK;
     } );
