@@ -54,8 +54,9 @@ enum uqc_layout { UQC_LAYOUT_REF = 0, UQC_LAYOUT_STATE_MAJOR = 1 };
  *            factor not positive definite, line-search or iteration limit)
  *            continue from their last accepted duals in the FP64 form. Where
  *            the FP64 form's kernel is the faster one it runs by default:
- *            systems "closure_tiny" takes, the 2-D Euler closure of up to 48 duals
- *            or without the tensor-core rounds, and its closure-only calls. */
+ *            systems "closure_tiny" takes, the 2-D Euler closure of up to 48 duals,
+ *            that without the tensor-core rounds except above 88 duals where the
+ *            mixed kernel holds three cells or more, and its closure-only calls. */
 enum uqc_precision { UQC_FP64 = 0, UQC_MIXED = 1 };
 
 /* Per-cell closure status (uqc_cell_status). */
@@ -166,9 +167,10 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
 /* Launch tuning (no reference counterpart; the autotuner uses it):
  *   "closure_group"  threads per cell in the closure kernel: 32 (a warp per
  *                    cell, several cells per CTA), 64 (two warps per cell,
- *                    up to four cells per CTA; the 2-D Euler closure: cells of
- *                    a CTA iterating together) or 256 (a CTA per cell);
- *                    0 = automatic.
+ *                    up to four cells per CTA; in FP64, where the system fits
+ *                    it, the batched kernel, a CTA's cells iterating together)
+ *                    or 256 (a CTA per cell); 0 = automatic: the batched kernel
+ *                    where it fits.
  *   "update_warps", "check_warps", "chord_warps"  warps (cells) per CTA of
  *                    the update kernel (default 8), the convergence-check
  *                    kernel (default 16) and the mixed form's chord kernel
@@ -213,7 +215,8 @@ int uqc_set_newton( uqc_solver* h, int max_iterations, double epsilon, int newto
  *                    on the tensor cores where its basis-pair table fits one
  *                    MMA (at most 256 pairs, i.e. total degree <= 5 in two
  *                    uncertainties) and the system has more than 48 duals, else
- *                    the FP64 form's kernel; 0 the single mixed kernel; 1 rounds with the CUDA-core Hessian; 2 rounds with
+ *                    the FP64 form's kernel or the single mixed kernel, whichever
+ *                    is faster; 0 the single mixed kernel; 1 rounds with the CUDA-core Hessian; 2 rounds with
  *                    the tensor-core Hessian (UQC_ERR_CONFIG where it does
  *                    not fit). Rounds: a chord kernel (a warp per cell, held
  *                    inverse H0^-1 in FP32, FP64 gradients and tests), then

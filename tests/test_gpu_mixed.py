@@ -125,3 +125,28 @@ def test_batch_larger_than_the_mesh(n):
     assert not sa.any() and not sb.any()
     # eps over the smallest eigenvalue of the Hessians (states in [4.5, 10.5]: DU above 1.5)
     np.testing.assert_allclose(lb, la, rtol=0, atol=2 * 1e-10 / 1.5)
+
+
+@pytest.mark.parametrize("degree,nquad,dim_xi,like", [
+    (6, 9, 2, "single"),     # 112 duals, the single kernel with four cells on an SM
+    (30, 64, 1, "single"),   # 124 duals, three
+    (6, 14, 2, "fp64"),      # 112 duals, 196 nodes: two
+    (4, 5, 3, "fp64"),       # 140 duals, two
+    (5, 12, 2, "fp64"),      # 84 duals: the batched kernel's smaller shape, at any count
+])
+def test_default_without_rounds(degree, nquad, dim_xi, like):
+    """Where the tensor-core rounds cannot run, the default is the single mixed
+    kernel or the FP64 form's, whichever is faster: its steps bit for bit."""
+    toml = W.euler2d(nx=10, ny=4, degree=degree, nquad=nquad, dim_xi=dim_xi, tend=10.0)
+    out = []
+    for options in ({}, {"precision": FP64} if like == "fp64" else {"mixed_hessian": 0}):
+        s = Solver(toml)
+        s.set_precision(options.get("precision", MIXED))
+        if "mixed_hessian" in options:
+            s.set_option("mixed_hessian", 0)
+        assert s.form()["mixed_form"] == 0 or like == "fp64"
+        s.init_state()
+        assert s.step(4)["failed_cells"] == 0
+        out.append(s.download_state())
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])

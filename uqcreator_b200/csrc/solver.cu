@@ -885,16 +885,24 @@ void plan_launches( uqc_solver* h ) {
     plan_mixed( h, maxSmem );
     plan_rounds( h, maxSmem );
     // Which kernel the mixed form's default runs on the 2-D Euler closure. Steps:
-    // k_newton where the tensor-core rounds cannot run, and up to 48 duals, where
-    // a step's eight or ten launches and an FP32 inverse gain nothing; closure-only
-    // calls (no held inverse): always. Closure phase of a warm step, mixed kernels /
-    // k_newton (us): 24 duals, 10k cells 153 / 59, 100k cells 293 / 193; 40 duals
-    // 205 / 100 and 443 / 425; 60 duals 272 / 229 and 642 / 1036; 84 duals 387 /
-    // 430 and, on 200k cells, 1460 / 5080; without rounds: 80 duals, 216 nodes 968
-    // / 801; 140 duals, 512 nodes 4553 / 3816 (first step 34193 / 17540). Any option
-    // that asks for the mixed kernels' form keeps them.
+    // k_newton up to 48 duals, where a step's eight or ten launches and an FP32
+    // inverse gain nothing on meshes of 10k to 100k cells (with 60 duals k_newton
+    // leads on the small mesh, the rounds on the large one: the line lies below them,
+    // the rounds' lead being the larger), and where the tensor-core rounds cannot run,
+    // unless its largest shape (two cells of an SM iterate, 16 warps) meets a single
+    // mixed kernel with three or four cells on an SM; closure-only calls (no held
+    // inverse): always. Closure phase of a warm step, mixed kernels / k_newton (us):
+    // 24 duals, 10k cells 153 / 59, 100k cells 293 / 193; 40 duals 205 / 100 and 443 /
+    // 425; 60 duals 272 / 229 and 642 / 1036; 84 duals 387 / 430 and, on 200k cells,
+    // 1460 / 5080. Without rounds, 100k cells (the single kernel's cells on an SM): 84
+    // duals, 144 nodes (4) 2764 / 2818, 256 nodes (2) 5979 / 4036; 112 duals, 81 nodes
+    // (4) 2956 / 4499, 144 nodes (3) 4445 / 5811, 196 nodes (2) 7028 / 6945, 576 nodes
+    // (2) 14943 / 13801; 140 duals, 216 nodes (3) 6556 / 7844, 512 nodes (2) 14694 /
+    // 14327 (its first step 242 / 126 ms). Any option that asks for the mixed kernels'
+    // form keeps them.
+    const bool singleLeads = h->newtonId == KERNEL_NEWTON_L2 && h->mixedOk && h->mixedBlock / h->mixedGroup >= 3;
     h->mixedNewtonOnce = h->newtonId && h->mixedOk && h->roundsOpt == -1 && h->chord && h->mixedMaxIter == 0;
-    h->mixedNewton     = h->mixedNewtonOnce && ( h->v2Mode == 0 || n <= 48 );
+    h->mixedNewton     = h->mixedNewtonOnce && ( ( h->v2Mode == 0 && !singleLeads ) || n <= 48 );
     if( h->deviceReady && h->precision == UQC_MIXED && ( wasForm != h->v2Mode || wasFp64 != h->mixedNewton || wasInverse != h->chordInverse ) ) {
         // another form: a store of its format, empty, and for the rounds a next-step
         // list with gradients
@@ -1140,7 +1148,7 @@ void launch_closure_fp64( uqc_solver* h, KParams& P, int mode ) {
 // length must be zero on entry (k_update resets them after every step).
 void launch_closure( uqc_solver* h, KParams& P, int mode ) {
     if( h->closureTiny && h->cfg.newtonMode != 2 ) {
-        // tiny systems: the FP64 register Newton in both precisions (the mixed
+        // tiny systems: k_newton_tiny, FP64 in both precisions (the mixed
         // form's FP32 Hessian saves nothing at this size)
         void* args[] = {&P, &mode};
         launch( h, pick( h->cfg.closure, h->tinyN, KERNEL_CLOSURE_TINY ), h->tinyGrid, 128, h->tinySmem, args );
