@@ -113,3 +113,12 @@ def test_sharded_solver_one_rank_over_nccl():
         ss.close()
     finally:
         dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("toml", [
+    W.burgers1d(ncells=40000, degree=9, nquad=40, tend=10.0),    # the whole mesh beyond the tiny kernel's size for 10 duals, a shard below it
+], ids=["burgers_10_duals"])
+def test_kernels_are_chosen_by_the_whole_mesh(toml):
+    """A shard runs the kernels that the whole mesh would, whatever its own size:
+    other kernels round differently."""
+    _compare(toml, 2, 4)

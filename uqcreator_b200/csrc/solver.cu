@@ -619,6 +619,10 @@ ClosureShape fp64_closure_shape( const uqc_solver* h, int maxSmem ) {
     return s;
 }
 
+// Cells that the rules of a plan go by: the whole mesh's for a shard too, so that it
+// runs the kernels, and rounds as, the unsharded handle.
+int plan_cells( const uqc_solver* h ) { return h->sharded ? h->shard.nGlobal : h->mesh.nCells; }
+
 // The batched Newton k_newton for the FP64 closure: the first shape whose cells
 // and CTAs per SM fit in shared memory and whose warps hold a CTA's row tiles
 // of 8 basis pairs. Small cells want many small CTAs (one warp a cell; their
@@ -795,7 +799,7 @@ void plan_launches( uqc_solver* h ) {
     // duals: Burgers, 500 cells 46 / 33, 20k cells 63 / 56 (first step 529 / 488), 200k cells
     // 361 / 377; shallow water, 50k cells, 48 / 43 but its first step 173 / 213
     h->closureTiny = h->tinyOpt != 0 && h->closureGroup == 32 && nQ <= TINY_MAX_NODES && !closure_linear( cl ) &&
-                     ( n <= size_t( TINY_N ) || ( n <= size_t( SMALL_N ) && ( h->tinyOpt == 1 || h->mesh.nCells <= SMALL_CELLS ) ) );
+                     ( n <= size_t( TINY_N ) || ( n <= size_t( SMALL_N ) && ( h->tinyOpt == 1 || plan_cells( h ) <= SMALL_CELLS ) ) );
     if( h->closureTiny ) {
         h->tinyN    = n <= size_t( TINY_N ) ? TINY_N : SMALL_N;
         void* kt    = pick( cl, h->tinyN, KERNEL_CLOSURE_TINY );
