@@ -156,7 +156,7 @@ def test_rounds_of_few_moments(degree, options):
     rounds, with the gradient they start from: the oracle's moments, and the
     Newton work of the check kernel's lists (update_test 0; the two gradients
     differ by rounding, which moves an iteration count in one cell of 10^5)."""
-    toml = W.euler2d(nx=24, ny=5, degree=degree, nquad=4)
+    toml = W.euler2d(nx=62, ny=20, degree=degree, nquad=4)    # more cells than a round of a warp each: the lanes' update
     o = Oracle(toml, W.mesh_for(toml))
     o.init_state()
     o.step(5)

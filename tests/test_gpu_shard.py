@@ -117,7 +117,11 @@ def test_sharded_solver_one_rank_over_nccl():
 
 @pytest.mark.parametrize("toml", [
     W.burgers1d(ncells=40000, degree=9, nquad=40, tend=10.0),    # the whole mesh beyond the tiny kernel's size for 10 duals, a shard below it
-], ids=["burgers_10_duals"])
+    # the whole mesh several rounds of the warp-per-cell update, a shard one: four lanes a cell
+    W.euler1d(ncells=9001, degree=4, nquad=10, tend=10.0),
+    W.euler2d(nx=41, ny=31, degree=2, nquad=4, tend=10.0),
+    W.euler2d(nx=33, ny=21, degree=3, nquad=6, tend=10.0),    # the whole mesh beyond a CTA an SM: two cells a warp
+], ids=["burgers_10_duals", "euler1d_5_moments", "euler2d_6_moments", "euler2d_10_moments"])
 def test_kernels_are_chosen_by_the_whole_mesh(toml):
     """A shard runs the kernels that the whole mesh would, whatever its own size:
     other kernels round differently."""

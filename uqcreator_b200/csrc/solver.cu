@@ -688,10 +688,15 @@ void plan_newton( uqc_solver* h, int maxSmem ) {
 // / k_update_mma, us: 10 moments, 36 nodes, 100k cells 351 / 223; 21 moments, 100
 // nodes, 200k cells 1150 / 811; 35 moments, 512 nodes, 262k cells 8950 / 5020): the
 // table whole where two CTAs' share of shared memory holds it beside the fluxes,
-// else in chunks of 64 nodes.
-void plan_update_mma( uqc_solver* h, int maxSmem ) {
+// else in chunks of 64 nodes. Not where two cells a warp leave the chip idle: at most
+// a CTA of 8 k_update warps an SM (k_update / k_update_mma, 600 cells: 10 moments, 36
+// nodes 18.5 / 18.6, 100 nodes 21.8 / 24.8; 21 moments, 196 nodes 30.6 / 35.0), or one
+// round of k_update (updRounds 1) with many nodes and one column tile of three in use
+// (6 moments, 100 nodes, 2,000 cells 23.7 / 25.4).
+void plan_update_mma( uqc_solver* h, int maxSmem, int updRounds ) {
     const int nT = h->tab.nT, nQ = h->tab.nQ, nQ4 = ( nQ + 3 ) & ~3;
     if( h->cfg.closure != 1 || h->d_bndNormal != nullptr || h->mesh.nFaces != 3 ) return;
+    if( plan_cells( h ) <= 8 * h->numSMs || ( nT <= 8 && nQ >= 64 && updRounds == 1 ) ) return;
     for( int tiles : UPD_TILES ) {
         if( nT > 8 * tiles ) continue;
         const int warps = h->updateWarpsOpt > 0 ? std::min( h->updateWarpsOpt, 8 ) : 8;
@@ -735,8 +740,20 @@ void plan_update_mma( uqc_solver* h, int maxSmem ) {
 // 2-D Euler, 6 moments, 10k cells 36 / 32, 100k 266 / 138 (k_update_mma 29 / 147; 3
 // moments 28 / 24 and 115 / 88, 10 moments, 100k cells 223 / 292: there a lane needs
 // all its registers and an SM holds eight warps).
-void plan_small( uqc_solver* h ) {
-    const int cl = h->cfg.closure, nT = h->tab.nT;
+// A lane takes a quarter of a cell's nodes here, a 32nd there, so a mesh that a warp
+// per cell covers in few rounds (updRounds, checkRounds) is the warps' when it has many
+// nodes: the rule compares nodes x (moments + 8) with a limit x rounds^2, the limits
+// per state count between the measured sides (update, us, warp / lanes; Burgers, 300
+// cells: 6 moments, 24 nodes 15.1 / 14.0, 96 nodes 13.9 / 18.3, 5,000 cells, 96 nodes 23 / 22;
+// shallow water, 300 cells, 10 moments, 20 nodes 1.01, 30 nodes 0.85 of the lanes' time;
+// 1-D Euler, 300 cells, 5 moments, 10 nodes 0.92, 70 nodes 18.4 / 35.0, 5,000 cells,
+// 30 nodes 1.03, 10,000 cells, 70 nodes 1.26). 2-D Euler: beyond 16 nodes, and beyond 4 in
+// one round, k_update_mma or k_update (6 moments, 16 / 100 nodes: 300 cells 0.76 / 0.33,
+// 100k cells 1.53 / 0.87 of the lanes' time).
+constexpr int UPDATE_LANES[3] = {600, 400, 70}, CHECK_LANES[3] = {250, 1500, 60};
+bool lanes_lead( int limit, int nT, int nQ, int rounds ) { return (long long)nQ * ( nT + 8 ) <= (long long)limit * rounds * rounds; }
+void plan_small( uqc_solver* h, int updRounds, int checkRounds ) {
+    const int cl = h->cfg.closure, nT = h->tab.nT, nQ = h->tab.nQ;
     if( h->d_bndNormal != nullptr || h->mesh.nFaces != ( h->nS == 4 ? 3 : 2 ) ) return;
     for( int ntm : SMALL_NT ) {
         if( nT > ntm ) continue;
@@ -750,7 +767,8 @@ void plan_small( uqc_solver* h ) {
             const int cells = block / LPC;
             grid            = std::min( std::max( 1, occ ) * h->numSMs, std::max( 1, ( h->mesh.nCells + cells - 1 ) / cells ) );
         };
-        if( void* fn = pick_small( cl, ntm, h->updateTests ? KERNEL_UPDATE_SMALL : KERNEL_UPDATE_SMALL_PLAIN ) ) {
+        const bool update = h->nS == 4 ? nQ <= ( updRounds == 1 ? 4 : 16 ) : lanes_lead( UPDATE_LANES[h->nS - 1], nT, nQ, updRounds );
+        if( void* fn = update ? pick_small( cl, ntm, h->updateTests ? KERNEL_UPDATE_SMALL : KERNEL_UPDATE_SMALL_PLAIN ) : nullptr ) {
             h->updateFn   = fn;
             h->updateSmem = table;
             shape( fn, table, h->updateWarpsOpt, h->updateBlock, h->updateGrid );
@@ -760,7 +778,9 @@ void plan_small( uqc_solver* h ) {
                 h->blockPartialCap = h->updateGrid;
             }
         }
-        if( void* fn = pick_small( cl, ntm, KERNEL_CHECK_SMALL ) ) {
+        // (no instance for four states; the one of 16 moments has its registers full)
+        const bool check = h->nS < 4 && lanes_lead( CHECK_LANES[h->nS - 1] / ( ntm == SMALL_NT[2] ? 4 : 1 ), nT, nQ, checkRounds );
+        if( void* fn = check ? pick_small( cl, ntm, KERNEL_CHECK_SMALL ) : nullptr ) {
             h->checkFn   = fn;
             h->checkSmem = 2 * table;
             shape( fn, 2 * table, h->checkWarpsOpt, h->checkBlock, h->checkGrid );
@@ -817,6 +837,7 @@ void plan_launches( uqc_solver* h ) {
         }
     }
     // update kernel: a warp per cell; phiWf + one node-flux buffer per warp
+    int updWarps = 0, checkWarps = 0;    // warps resident on the device
     {
         const size_t uTables = h->tablesInSmem ? ( ( size_t( nQ ) * h->ld + 4 + 3 ) & ~size_t( 3 ) ) * sizeof( double ) : 0;
         const size_t perWarp = update_warp_doubles( nS, nQ, h->mesh.nFaces ) * sizeof( double );
@@ -849,6 +870,7 @@ void plan_launches( uqc_solver* h ) {
         // in registers, so in CTAs per SM)
         CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, ku, h->updateBlock, h->updateSmem ) );
         h->updateGrid = std::max( 1, occ ) * h->numSMs;
+        updWarps      = h->updateGrid * warps;
         h->updateGrid = std::min( h->updateGrid, std::max( 1, ( h->mesh.nCells + warps - 1 ) / warps ) );
         // one residual partial per CTA of k_update (grows with the grid; a
         // re-plan waits for the device in cudaFree before replacing it)
@@ -879,10 +901,13 @@ void plan_launches( uqc_solver* h ) {
         h->checkFn    = kk;
         allow_dynamic_smem( kk );
         CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, kk, h->checkBlock, h->checkSmem ) );
+        checkWarps   = std::max( 1, occ ) * h->numSMs * warps;
         h->checkGrid = std::min( std::max( 1, occ ) * h->numSMs, std::max( 1, ( h->mesh.nCells + warps - 1 ) / warps ) );
     }
-    plan_update_mma( h, maxSmem );
-    plan_small( h );
+    // rounds that the warp-per-cell kernels planned so far take over the mesh
+    const int updRounds = ( plan_cells( h ) + updWarps - 1 ) / updWarps, checkRounds = ( plan_cells( h ) + checkWarps - 1 ) / checkWarps;
+    plan_update_mma( h, maxSmem, updRounds );
+    plan_small( h, updRounds, checkRounds );
     plan_newton( h, maxSmem );
     const int wasForm  = h->v2Mode;
     const bool wasFp64 = h->mixedNewton, wasInverse = h->chordInverse;
