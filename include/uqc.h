@@ -56,7 +56,8 @@ enum uqc_layout { UQC_LAYOUT_REF = 0, UQC_LAYOUT_STATE_MAJOR = 1 };
  *            the FP64 form's kernel is the faster one it runs by default:
  *            systems "closure_tiny" takes, the 2-D Euler closure of up to 48 duals,
  *            that without the tensor-core rounds except above 88 duals where the
- *            mixed kernel holds three cells or more, and its closure-only calls. */
+ *            mixed kernel holds three cells or more, the closures of one and two
+ *            states, and closure-only calls. */
 enum uqc_precision { UQC_FP64 = 0, UQC_MIXED = 1 };
 
 /* Per-cell closure status (uqc_cell_status). */

@@ -150,3 +150,24 @@ def test_default_without_rounds(degree, nquad, dim_xi, like):
         out.append(s.download_state())
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("toml,like", [
+    (W.euler1d(ncells=90, degree=4, nquad=10, tend=10.0), "single"),
+    (W.burgers1d(ncells=90, degree=11, nquad=32, tend=10.0), "fp64"),
+    (W.shallow_water1d(ncells=90, max_degree=8, nquad=20, tend=10.0), "fp64"),
+], ids=["euler1d", "burgers", "sw"])
+def test_default_of_other_closures(toml, like):
+    """One and two states run the FP64 form's kernel by default, three the single
+    mixed kernel, whichever is faster: its steps bit for bit."""
+    out = []
+    for options in ({}, {"precision": FP64} if like == "fp64" else {"mixed_hessian": 0}):
+        s = Solver(toml)
+        s.set_precision(options.get("precision", MIXED))
+        if "mixed_hessian" in options:
+            s.set_option("mixed_hessian", 0)
+        s.init_state()
+        assert s.step(6)["failed_cells"] == 0
+        out.append(s.download_state())
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])

@@ -743,13 +743,13 @@ void plan_update_mma( uqc_solver* h, int maxSmem, int updRounds ) {
 // A lane takes a quarter of a cell's nodes here, a 32nd there, so a mesh that a warp
 // per cell covers in few rounds (updRounds, checkRounds) is the warps' when it has many
 // nodes: the rule compares nodes x (moments + 8) with a limit x rounds^2, the limits
-// per state count between the measured sides (update, us, warp / lanes; Burgers, 300
-// cells: 6 moments, 24 nodes 15.1 / 14.0, 96 nodes 13.9 / 18.3, 5,000 cells, 96 nodes 23 / 22;
-// shallow water, 300 cells, 10 moments, 20 nodes 1.01, 30 nodes 0.85 of the lanes' time;
-// 1-D Euler, 300 cells, 5 moments, 10 nodes 0.92, 70 nodes 18.4 / 35.0, 5,000 cells,
-// 30 nodes 1.03, 10,000 cells, 70 nodes 1.26). 2-D Euler: beyond 16 nodes, and beyond 4 in
-// one round, k_update_mma or k_update (6 moments, 16 / 100 nodes: 300 cells 0.76 / 0.33,
-// 100k cells 1.53 / 0.87 of the lanes' time).
+// per state count between the measured sides (update, us, warp / lanes; Burgers, 6
+// moments: 300 cells, 24 nodes 14.5 / 13.2, 96 nodes 15.2 / 20.1, 5,000 cells, 96 nodes
+// 22.2 / 21.3; shallow water, 10 moments, 300 cells, 20 nodes 14.1 / 14.0, 30 nodes 13.7 /
+// 16.1; 1-D Euler, 5 moments: 300 cells, 10 nodes 15.7 / 17.1, 70 nodes 17.2 / 32.9, 5,000
+// cells, 30 nodes 24.6 / 23.9, 10,000 cells, 70 nodes 46.0 / 36.6). 2-D Euler: beyond 16
+// nodes, and beyond 4 in one round, k_update_mma or k_update (6 moments, 16 nodes: 288
+// cells 16.2 / 21.6, 50k cells 110.7 / 71.7; 100 nodes 19.6 / 59.3 and 261 / 383).
 constexpr int UPDATE_LANES[3] = {600, 400, 70}, CHECK_LANES[3] = {250, 1500, 60};
 bool lanes_lead( int limit, int nT, int nQ, int rounds ) { return (long long)nQ * ( nT + 8 ) <= (long long)limit * rounds * rounds; }
 void plan_small( uqc_solver* h, int updRounds, int checkRounds ) {
@@ -913,7 +913,7 @@ void plan_launches( uqc_solver* h ) {
     const bool wasFp64 = h->mixedNewton, wasInverse = h->chordInverse;
     plan_mixed( h, maxSmem );
     plan_rounds( h, maxSmem );
-    // Which kernel the mixed form's default runs on the 2-D Euler closure. Steps:
+    // Which kernel the mixed form's default runs. 2-D Euler closure, steps:
     // k_newton up to 48 duals, where a step's eight or ten launches and an FP32
     // inverse gain nothing on meshes of 10k to 100k cells (with 60 duals k_newton
     // leads on the small mesh, the rounds on the large one: the line lies below them,
@@ -927,11 +927,14 @@ void plan_launches( uqc_solver* h ) {
     // duals, 144 nodes (4) 2764 / 2818, 256 nodes (2) 5979 / 4036; 112 duals, 81 nodes
     // (4) 2956 / 4499, 144 nodes (3) 4445 / 5811, 196 nodes (2) 7028 / 6945, 576 nodes
     // (2) 14943 / 13801; 140 duals, 216 nodes (3) 6556 / 7844, 512 nodes (2) 14694 /
-    // 14327 (its first step 242 / 126 ms). Any option that asks for the mixed kernels'
-    // form keeps them.
+    // 14327 (its first step 242 / 126 ms). One and two states: k_newton (30k cells: Burgers,
+    // 11 duals 134 / 99; shallow water, 20 duals 88 / 54). Three: the single kernel, whose
+    // half as many more iterations with a held factor cost less (1-D Euler, 300k cells:
+    // 15 duals 66 / 80, 39 duals 90 / 103; two uncertainties, 30 duals 100 / 133). Any option that
+    // asks for the mixed kernels' form keeps them.
     const bool singleLeads = h->newtonId == KERNEL_NEWTON_L2 && h->mixedOk && h->mixedBlock / h->mixedGroup >= 3;
     h->mixedNewtonOnce = h->newtonId && h->mixedOk && h->roundsOpt == -1 && h->chord && h->mixedMaxIter == 0;
-    h->mixedNewton     = h->mixedNewtonOnce && ( ( h->v2Mode == 0 && !singleLeads ) || n <= 48 );
+    h->mixedNewton     = h->mixedNewtonOnce && nS != 3 && ( ( h->v2Mode == 0 && !singleLeads ) || n <= 48 );
     if( h->deviceReady && h->precision == UQC_MIXED && ( wasForm != h->v2Mode || wasFp64 != h->mixedNewton || wasInverse != h->chordInverse ) ) {
         // another form: a store of its format, empty, and for the rounds a next-step
         // list with gradients
