@@ -214,3 +214,22 @@ def test_register_newton_matches_oracle_and_general_kernel(toml, steps):
     np.testing.assert_array_equal(vs, o.get_state()[2])
     np.testing.assert_array_equal(vs, vg)
     np.testing.assert_allclose(us, ug, rtol=1e-9, atol=1e-11)
+
+
+@pytest.mark.parametrize("n", [1, 20, 300, 2000])
+def test_host_closure_layouts_agree(n):
+    """Batches on pinned memory, through two copies of the reference layout's
+    arrays, and through one: the same duals in both layouts, the caller's
+    moments untouched."""
+    toml = W.euler2d(nx=40, ny=25, degree=3, nquad=6)
+    s = Solver(toml)
+    s.init_state()
+    u, lam, _ = s.download_state()
+    u, lam = u[-n:].copy(), lam[-n:].copy()
+    a, sa = s.closure_solve_host(lam, u)
+    ur, lr = (np.ascontiguousarray(x.transpose(0, 2, 1)) for x in (u, lam))
+    keep = ur.copy()
+    b, sb = s.closure_solve_host(lr.reshape(u.shape), ur.reshape(u.shape), layout=LAYOUT_REF)
+    np.testing.assert_array_equal(sa, sb)
+    np.testing.assert_array_equal(b.reshape(lr.shape).transpose(0, 2, 1), a)
+    np.testing.assert_array_equal(ur, keep)
