@@ -973,8 +973,9 @@ template <int CL> __global__ void __launch_bounds__( 512, 1 ) k_invert_sweep( KP
                 const float p00 = pr0[32 * CW], p01 = pr1[32 * CW], p11 = pr1[32 * CW + 1];
                 const float det = fmaf( p00, p11, -p01 * p01 );
                 // not positive definite, or entries above 1e19, whose product FP32 does not hold (the
-                // sweep's e - P^-1 e has lost such a block's inverse in any case)
-                bad             = bad || !( p00 > 0.f && det > 0.f && isfinite( det ) );
+                // sweep's e - P^-1 e has lost such a block's inverse in any case); by the bits, a NaN
+                // being neither
+                bad             = bad || __float_as_int( p00 ) <= 0 || unsigned( __float_as_int( det ) - 1 ) >= 0x7F7FFFFFu;
                 const float r   = __frcp_rn( det );
                 const float i00 = p11 * r, i01 = -p01 * r, i11 = p00 * r;
                 // w = P^-1 v of this thread's columns

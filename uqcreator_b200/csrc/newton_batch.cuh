@@ -29,11 +29,11 @@
 // What bounds it: with 140 duals and 512 nodes the product (61 % of a cell's
 // cycles, at 75 % of the FP64 rate); with 84 duals and 100 nodes the dependent
 // chain of the elimination (40 %), which the other cells of the SM only partly
-// cover (four cells fit: 35 KB of Hessian each); FP64 pipe 30-45 % busy. Cycles
-// of one cell's iteration on an SM (its share of them): 43,000 in k_closure
-// (four cells of two warps each) -> 21,000 with 84 duals, 420,000 -> 140,000
-// with 140; 2-D Euler, 200k cells, closure phase of a step 10.2 -> 5.1 ms; 262k
-// cells, three uncertainties, 88.5 -> 31 ms.
+// cover (four cells fit: 41 KB each, 34 KB of it Hessian, and a 17 KB table per
+// CTA); FP64 pipe 30-45 % busy. Cycles of one cell's iteration on an SM (its share
+// of them): 43,000 in k_closure (four cells of two warps each) -> 21,000 with 84
+// duals, 420,000 -> 140,000 with 140; 2-D Euler, 200k cells, closure phase of a step
+// 10.2 -> 5.1 ms; 262k cells, three uncertainties, 88.5 -> 31 ms.
 #pragma once
 #include "chord.cuh"
 
@@ -126,7 +126,9 @@ __device__ __forceinline__ bool tile_sweep( double& c0, double& c1, int lane ) {
 
 // The sweep of S T S, S the powers of two that take T's diagonal entries to [1, 4):
 // the determinants of entries beyond 2^+-500 leave the format's range (or the
-// reciprocal's) although the entries do not. D <- -S (S T S)^-1 S.
+// reciprocal's) although the entries do not. D <- -S (S T S)^-1 S. (A call that no usual
+// state takes; its being there costs the others 0.5 %: closure phase of a warm step, 200k
+// cells of 84 duals, 3.553 -> 3.570 ms; inlined 0.7 %, as a second round of a loop 3 %.)
 static __device__ __noinline__ bool tile_sweep_scaled( double* D, double c0, double c1, int lane ) {
     const unsigned full = 0xffffffffu;
     const int g = lane >> 2, t = lane & 3;
@@ -144,7 +146,7 @@ static __device__ __noinline__ bool tile_sweep_scaled( double* D, double c0, dou
 // D <- -T^-1 (see tile_sweep); returns false if T is not positive definite.
 __device__ __forceinline__ bool tile_sweep_inverse( double* D, double c0, double c1, int lane ) {
     double x0 = c0, x1 = c1;
-    if( !tile_sweep( x0, x1, lane ) ) return tile_sweep_scaled( D, c0, c1, lane );
+    if( __builtin_expect( !tile_sweep( x0, x1, lane ), 0 ) ) return tile_sweep_scaled( D, c0, c1, lane );
     *reinterpret_cast<double2*>( D + rix( lane >> 2, 2 * ( lane & 3 ) ) ) = make_double2( x0, x1 );
     return true;
 }
