@@ -84,7 +84,8 @@ FACTOR_UNIT = {"fp64": "fp64", "mixed": "fp32"}
 # DRAM bytes (read + write) of the closure phase per cell that takes Newton
 # iterations, from ncu captures of the 5th step of a 60,000-cell case of the
 # same workload (6,457 active cells; profiles/closure_rounds_euler2d.md):
-# FP64 form k_closure 9.58 MB; mixed form (rounds) k_chord rounds 0-1, k_hess_tc
+# FP64 form k_closure 9.58 MB (k_newton, which replaced it, 9.5 MB: 6.6 GB/s over
+# 1.44 ms, profiles/newton_and_updates_current.md); mixed form (rounds) k_chord rounds 0-1, k_hess_tc
 # and k_invert_sweep round 0: 358.9 MB, mostly each active cell's held FP32
 # inverse (28 KB) read by the chord kernel.
 CLOSURE_DRAM_BYTES_PER_ACTIVE_CELL = {"fp64": 9.576e6 / 6457, "mixed": 358.9e6 / 6457}
@@ -116,7 +117,7 @@ def closure_roofline(form, n_states, n_total, n_quad, cells, steps, ref_info, cl
             "traffic_unit": "bytes per closure phase (scaled from the form's ncu capture by its active cells)",
             "t_bound_ms": t_unit, "closure_ms_per_launch": closure_ms, "flops_per_launch": total,
             "peaks_tflops": {**peak, "tensor_source": f"bf16 {src} (MEASURED_PEAKS.json)"},
-            "hbm_peak_gbs": hbm, "kernels": "closure phase: k_check + k_closure (FP64 form); k_check + k_chord / k_hess_tc / k_invert_sweep rounds + the FP64 fallback pass (mixed form)"}
+            "hbm_peak_gbs": hbm, "kernels": "closure phase: k_check + k_newton (FP64 form); k_check + k_chord / k_hess_tc / k_invert_sweep rounds + the FP64 fallback pass (mixed form)"}
 
 
 class Clocks:

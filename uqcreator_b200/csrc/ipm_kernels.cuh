@@ -1,7 +1,9 @@
 // FP64 kernels of the IPM time step.
 //
-//   k_closure  persistent, work-stealing (k_newton of newton_batch.cuh replaces
-//              it for the 2-D Euler closure): one thread group (a warp for small
+//   k_closure  persistent, work-stealing (k_newton of newton_batch.cuh and
+//              k_newton_tiny replace it in FP64 for every nonlinear closure whose
+//              system fits theirs, but not for SolveClosureSafe or the One-Shot
+//              step): one thread group (a warp for small
 //              systems, a whole CTA for n = nS nT > 32) per cell. Runs the
 //              damped Newton of Closure::SolveClosure (closure.cpp:133-193) with
 //              the basis tables staged in shared memory, the Hessian kept in
@@ -111,7 +113,7 @@ struct KParams {
     const float* phiF;       // nQ x ld: phi rounded to FP32 (mixed form)
     const double* phiT;      // nT x ldT: phi node-contiguous, zero from nQ to ldT (k_newton)
     int ldT;                 // nQ rounded up to 4
-    const double* tinyTab;   // k_newton_tiny: nQ x 32, column e the table of its sum e
+    const double* tinyTab;   // k_newton_tiny: nQ x tiny_cols(N) (32 or 96), column e the table of its sum e
     const double* phiWfP;    // k_update_mma: phiWf padded with zeros, nQ rounded up to 4 rows of ldP
     int ldP;
     int updNodes;            // k_update_mma: nodes per chunk (a multiple of 4; all of them: the table stays)

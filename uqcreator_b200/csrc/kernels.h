@@ -25,10 +25,10 @@ enum KernelId {
     KERNEL_CLOSURE_TINY      = 15,   // k_newton_tiny
     KERNEL_UPDATE_SPLIT      = 16,   // k_update (with / without the test) whose projection splits
     KERNEL_UPDATE_PLAIN_SPLIT = 17,  // the nodes of a small last block of basis functions
-    KERNEL_NEWTON_S4          = 18,  // k_newton (2-D Euler): 4 cells on 4 warps, 4 CTAs per SM, at most 8 row tiles of pairs
+    KERNEL_NEWTON_S4          = 18,  // k_newton (nonlinear closures): 4 cells on 4 warps, 4 CTAs per SM, at most 8 row tiles of pairs
     KERNEL_NEWTON_S2          = 19,  // ... 2 cells on 4 warps, 4 CTAs per SM, at most 16
-    KERNEL_NEWTON_M2          = 20,  // ... 2 cells on 8 warps, 2 CTAs per SM, at most 32
-    KERNEL_NEWTON_L2          = 21,  // ... 2 cells on 16 warps, at most 80
+    KERNEL_NEWTON_M2          = 20,  // ... (2-D Euler) 2 cells on 8 warps, 2 CTAs per SM, at most 32
+    KERNEL_NEWTON_L2          = 21,  // ... (2-D Euler) 2 cells on 16 warps, at most 80
     KERNEL_CHECK_SMALL        = 22,  // k_check_small (group: its NTM), nonlinear closures
     KERNEL_UPDATE_SMALL       = 23,  // k_update_small with / without the next step's test (group: NTM)
     KERNEL_UPDATE_SMALL_PLAIN = 24,

@@ -144,7 +144,7 @@ template <int CL, int NTM> __global__ void __launch_bounds__( 256, 2 ) k_check_s
         int newLev = lev;
         if( P.nLevels > 1 ) newLev = level_rule( P, level_indicator( P, [&]( int i ) { return uh[i]; }, lev, nTj ), lev );
         const int nTn = P.nTLevel[newLev];
-        // loop bound of the warp's four cells
+        // loop bound of the warp's cells
         const int nMax = __reduce_max_sync( 0xffffffffu, max( nTj, nTn ) );
         double l[NS][NTM], acc[NS][NTM];
 #pragma unroll
